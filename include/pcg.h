@@ -38,7 +38,7 @@ enum {
     PCG_ERR_BUDGET = 5,      /* request does not fit the serving memory budget */
     PCG_ERR_NOT_FOUND = 6,   /* unknown request id */
     PCG_ERR_NOT_READY = 7,   /* request not finished yet */
-    PCG_ERR_DEVICE = 8       /* a kernel stopped early (bounded wait ran out, unaligned copy refused) */
+    PCG_ERR_DEVICE = 8       /* a kernel stopped early (bounded wait ran out) */
 };
 
 /* Same layout as GridParams (shaders/types.h:23-37). */

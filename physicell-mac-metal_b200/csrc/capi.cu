@@ -195,8 +195,7 @@ pcg_status pcg_sync(pcg_ctx* ctx)
     if (st) {
         PCG_CU(ctx, cudaMemsetAsync(ctx->status, 0, sizeof st, ctx->stream));
         PCG_CU(ctx, cudaStreamSynchronize(ctx->stream));
-        return fail(ctx, PCG_ERR_DEVICE, std::string("a kernel stopped early:") + ((st & PCG_DEV_TIMEOUT) ? " wait limit reached" : "") +
-                                              ((st & PCG_DEV_ALIGN) ? " unaligned bulk copy refused" : ""));
+        return fail(ctx, PCG_ERR_DEVICE, "a kernel stopped early: wait limit reached");
     }
     return PCG_OK;
 }

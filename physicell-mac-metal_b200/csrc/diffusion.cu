@@ -28,9 +28,8 @@
 //             4 values per 16-byte shared access, coefficients broadcast;
 //   y/z tile: 32 adjacent columns x n rows stored [row][32] (3-D map, box
 //             32 x n); lane = column.
-// Lines too long for a tensor box move with 1-D bulk copies (x: the whole
-// tile, lanes skewed by the lane index so 32 lanes hit 32 banks; y/z: one
-// 128-byte copy per row).
+// Lines too long for a tensor box are solved by one warp each, as scans of
+// the two affine recurrences over the warp's lanes (k_sweep_long).
 // Every value is read from HBM once and written once per sweep.  Waits are
 // bounded: a wait that runs out records PCG_DEV_TIMEOUT in the status word,
 // drains what it issued, and returns.
@@ -130,13 +129,6 @@ __device__ __forceinline__ void bulk_load(void* smem_dst, const void* gsrc, uint
                  : "memory");
 }
 
-// shared -> global in this thread's bulk group
-__device__ __forceinline__ void bulk_store(void* gdst, const void* smem_src, uint32_t bytes)
-{
-    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gdst), "r"(smem_u32(smem_src)),
-                 "r"(bytes)
-                 : "memory");
-}
 // 3-D tensor-map copies of a whole column tile (one instruction each way)
 __device__ __forceinline__ void tensor_load3(void* smem_dst, const void* tmap, int c0, int c1, int c2, uint64_t* bar)
 {
@@ -186,17 +178,8 @@ __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.w
 __device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ void fence_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
-__device__ __forceinline__ bool aligned16(const void* p, uint32_t bytes)
-{
-    return ((reinterpret_cast<uintptr_t>(p) | bytes) & 15u) == 0 && bytes > 0;
-}
-
 // ------------------------------------------------------------------ tile geometry
 
-// Bytes of one row copy of a column tile (count columns rounded up to 4).
-__device__ __forceinline__ uint32_t col_row_bytes(uint32_t count) { return ((count + 3u) & ~3u) * 4u; }
-
-// Issue the loads of 'tile' into stage 'st' (all lanes take part).
 // Tensor coordinates of a column tile's box: (x, slab, line position).
 __device__ __forceinline__ void tile_coords(const SweepTile& tile, int* c)
 {
@@ -205,100 +188,42 @@ __device__ __forceinline__ void tile_coords(const SweepTile& tile, int* c)
     c[2] = 0;
 }
 
-// Issue the loads of 'tile' into stage 'st' and of its rule's coefficient
-// table into 'stab' (the stage's table area), all counted on 'bar'.
+// Issue (lane 0) the load of 'tile' into stage 'st' and of its rule's
+// coefficient table into 'stab' (the stage's table area), both counted on
+// 'bar'.
 template <bool kRows>
-__device__ __forceinline__ bool issue_tile_load(const SweepTile& tile, const float* __restrict__ dens,
-                                                const float* __restrict__ tab, const void* tmaps, float* st,
-                                                float* stab, uint64_t* bar, int lane, unsigned* status)
+__device__ __forceinline__ void issue_tile_load(const SweepTile& tile, const float* __restrict__ tab, const void* tmaps,
+                                                float* st, float* stab, uint64_t* bar, int lane)
 {
-    const LineRule r = rule_of(tile);
-    const uint32_t n = r.n;
+    if (lane != 0) return;
+    const uint32_t n = tile.n;
     const uint32_t tb = tab_floats(n) * 4u;    // 32-byte multiple, 32-byte aligned source
-    const float* src = dens + tile.base;
     const void* map = static_cast<const unsigned char*>(tmaps) + static_cast<size_t>(tile.map) * 128;
-    if (kRows && (tile.face & TILE_TENSOR)) {
-        if (lane == 0) {
-            mbar_arrive_expect_tx(bar, 32u * row_smem_pitch(n) * 4u + tb);   // the whole box, fill included
-            tensor_load2(st, map, 0, static_cast<int>(tile.outer), bar);
-            bulk_load(stab, tab + r.tab, tb, bar);
-        }
-        return true;
-    }
-    if (!kRows && (tile.face & TILE_TENSOR)) {
-        if (lane == 0) {
-            int c[3];
-            tile_coords(tile, c);
-            mbar_arrive_expect_tx(bar, 32u * n * 4u + tb);
-            tensor_load3(st, map, c[0], c[1], c[2], bar);
-            bulk_load(stab, tab + r.tab, tb, bar);
-        }
-        return true;
-    }
     if (kRows) {
-        const uint32_t bytes = tile.count * tile.rs * 4u;     // count lines of pitch rs
-        if (lane == 0) {
-            if (!aligned16(src, bytes)) {
-                atomicOr(status, PCG_DEV_ALIGN);
-                mbar_arrive_expect_tx(bar, 0);
-                return false;
-            }
-            mbar_arrive_expect_tx(bar, bytes + tb);
-            bulk_load(st, src, bytes, bar);
-            bulk_load(stab, tab + r.tab, tb, bar);
-        }
+        mbar_arrive_expect_tx(bar, 32u * row_smem_pitch(n) * 4u + tb);   // the whole box, fill included
+        tensor_load2(st, map, 0, static_cast<int>(tile.outer), bar);
     } else {
-        const uint32_t rb = col_row_bytes(tile.count);
-        if (!aligned16(src, rb) || (tile.rs & 3u)) {
-            if (lane == 0) {
-                atomicOr(status, PCG_DEV_ALIGN);
-                mbar_arrive_expect_tx(bar, 0);
-            }
-            return false;
-        }
-        if (lane == 0) {
-            mbar_arrive_expect_tx(bar, rb * n + tb);
-            bulk_load(stab, tab + r.tab, tb, bar);
-        }
-        __syncwarp();
-        for (uint32_t j = lane; j < n; j += 32) bulk_load(st + j * 32, src + static_cast<size_t>(j) * tile.rs, rb, bar);
+        int c[3];
+        tile_coords(tile, c);
+        mbar_arrive_expect_tx(bar, 32u * n * 4u + tb);
+        tensor_load3(st, map, c[0], c[1], c[2], bar);
     }
-    return true;
+    bulk_load(stab, tab + tile.tab, tb, bar);
 }
 
 template <bool kRows>
-__device__ __forceinline__ void issue_tile_store(const SweepTile& tile, float* __restrict__ dens, const void* tmaps, const float* st, int lane)
+__device__ __forceinline__ void issue_tile_store(const SweepTile& tile, const void* tmaps, const float* st, int lane)
 {
-    float* dst = dens + tile.base;
-    if (kRows && (tile.face & TILE_TENSOR)) {
-        if (lane == 0) {
-            tensor_store2(static_cast<const unsigned char*>(tmaps) + static_cast<size_t>(tile.map) * 128, 0,
-                          static_cast<int>(tile.outer), st);
-            bulk_commit();
-        }
-        return;
-    }
-    if (!kRows && (tile.face & TILE_TENSOR)) {
-        if (lane == 0) {
-            int c[3];
-            tile_coords(tile, c);
-            tensor_store3(static_cast<const unsigned char*>(tmaps) + static_cast<size_t>(tile.map) * 128, c[0], c[1],
-                          c[2], st);
-            bulk_commit();
-        }
-        return;
-    }
+    if (lane != 0) return;
+    const void* map = static_cast<const unsigned char*>(tmaps) + static_cast<size_t>(tile.map) * 128;
     if (kRows) {
-        if (lane == 0) {
-            bulk_store(dst, st, tile.count * tile.rs * 4u);
-            bulk_commit();
-        }
+        tensor_store2(map, 0, static_cast<int>(tile.outer), st);
     } else {
-        const uint32_t n = tile.n;
-        const uint32_t rb = col_row_bytes(tile.count);
-        for (uint32_t j = lane; j < n; j += 32) bulk_store(dst + static_cast<size_t>(j) * tile.rs, st + j * 32, rb);
-        bulk_commit();
+        int c[3];
+        tile_coords(tile, c);
+        tensor_store3(map, c[0], c[1], c[2], st);
     }
+    bulk_commit();
 }
 
 // ------------------------------------------------------------------ solves in shared memory
@@ -466,8 +391,7 @@ __device__ __forceinline__ void row_line(float* row, const LineRule& r, const fl
     }
 }
 
-__device__ __forceinline__ void solve_rows_vec(float* st, const LineRule& r, const float* t, int lane,
-                                               int count)
+__device__ __forceinline__ void solve_rows(float* st, const LineRule& r, const float* t, int lane, int count)
 {
     if (lane >= count) return;
     row_line(st + lane * static_cast<int>(row_smem_pitch(r.n)), r, t);
@@ -505,67 +429,6 @@ __device__ __forceinline__ void solve_cols(float* st, const SweepTile& tile, con
     }
 }
 
-// x tile moved as one 1-D bulk copy (lines longer than a tensor box): lane t
-// solves line t stored at st + t * px.  Lane t reaches interior position i
-// at step i + t, so at every step the 32 lanes touch 32 different banks
-// (px is a multiple of 4, so px - 1 is odd).
-__device__ __forceinline__ void skew_step_fwd(float* p, const float* t, int i, float& d)
-{
-    d = fmaf(tab_g(t, i + 1), d, p[i] * tab_inv(t, i + 1));
-    p[i] = d;
-}
-__device__ __forceinline__ void skew_step_bwd(float* p, const float* t, int i, float& x)
-{
-    x = fmaf(tab_g(t, i + 1), x, p[i]);
-    p[i] = x;
-}
-
-__device__ __forceinline__ void solve_rows(float* st, const SweepTile& tile, const LineRule& r, const float* t,
-                                           int lane)
-{
-    const int n = static_cast<int>(r.n);
-    const int px = static_cast<int>(tile.rs);
-    const bool act = lane < static_cast<int>(tile.count);
-    float* row = st + lane * px;
-    if (n >= 3) {
-        const int m = n - 2;
-        float* p = row + 1;   // interior position i + 1 at p[i]
-        if (act) {
-            p[0] += r.fold;
-            if (m > 1) p[m - 1] += r.fold;
-        }
-        // steps [0, 31) and [max(m, 31), m + 31) are predicated, [31, m) is
-        // taken by every lane
-        const int c_begin = m > 31 ? m : 31;
-        float d = 0.f;
-        for (int k = 0; k < 31; ++k) {
-            const int i = k - lane;
-            if (i >= 0 && i < m) skew_step_fwd(p, t, i, d);
-        }
-#pragma unroll 4
-        for (int k = 31; k < m; ++k) skew_step_fwd(p, t, k - lane, d);
-        for (int k = c_begin; k < m + 31; ++k) {
-            const int i = k - lane;
-            if (i >= 0 && i < m) skew_step_fwd(p, t, i, d);
-        }
-        float x = 0.f;
-        for (int k = 0; k < 31; ++k) {
-            const int i = m - 1 - (k - lane);
-            if (i >= 0 && i < m) skew_step_bwd(p, t, i, x);
-        }
-#pragma unroll 4
-        for (int k = 31; k < m; ++k) skew_step_bwd(p, t, m - 1 - (k - lane), x);
-        for (int k = c_begin; k < m + 31; ++k) {
-            const int i = m - 1 - (k - lane);
-            if (i >= 0 && i < m) skew_step_bwd(p, t, i, x);
-        }
-    }
-    if (act && r.dir) {
-        row[0] = r.T;
-        row[n - 1] = r.T;
-    }
-}
-
 // ------------------------------------------------------------------ pipelined kernel
 
 // Shared memory: kBarBytes of mbarriers ([warp][stage]), then the stages
@@ -582,10 +445,9 @@ __host__ __device__ constexpr int sweep_header_bytes(int warps, int nstages)
 }
 
 template <bool kRows>
-__global__ void __launch_bounds__(256, 1) k_sweep_tma(float* __restrict__ dens, const SweepTile* __restrict__ tiles,
-                                                   uint32_t ntiles, const float* __restrict__ tab,
-                                                   const void* __restrict__ tmaps, int stage_floats, int nstages,
-                                                   int tab_area, int apply_faces,
+__global__ void __launch_bounds__(256, 1) k_sweep_tma(const SweepTile* __restrict__ tiles, uint32_t ntiles,
+                                                   const float* __restrict__ tab, const void* __restrict__ tmaps,
+                                                   int stage_floats, int nstages, int tab_area, int apply_faces,
                                                    const uint8_t* __restrict__ mask, unsigned* __restrict__ status)
 {
     // stage: [tile data][tab_area floats of coefficient table]
@@ -612,7 +474,7 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tma(float* __restrict__ dens, 
     auto issue = [&]() {
         const int s = static_cast<int>(issued % nstages);
         float* st = stages + s * stage_floats;
-        issue_tile_load<kRows>(nd, dens, tab, tmaps, st, st + stage_floats - tab_area, &bars[s], lane, status);
+        issue_tile_load<kRows>(nd, tab, tmaps, st, st + stage_floats - tab_area, &bars[s], lane);
         if (lane == 0) descs[s] = nd;
         ++issued;
         if (issued < ntw) nd = tiles[gw + issued * tw];
@@ -638,15 +500,14 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tma(float* __restrict__ dens, 
         const float* t = st + stage_floats - tab_area;
         if (tile_on(r, mask)) {
             if (kRows) {
-                if (tile.face & TILE_TENSOR) solve_rows_vec(st, r, t, lane, static_cast<int>(tile.count));
-                else solve_rows(st, tile, r, t, lane);
+                solve_rows(st, r, t, lane, static_cast<int>(tile.count));
             } else {
                 solve_cols(st, tile, r, t, lane, apply_faces != 0);
             }
         }
         fence_async_smem();
         __syncwarp();
-        issue_tile_store<kRows>(tile, dens, tmaps, st, lane);
+        issue_tile_store<kRows>(tile, tmaps, st, lane);
     }
     if (!ok) {
         // let every load this warp issued land before the CTA exits (bounded)
@@ -788,52 +649,159 @@ __global__ void __launch_bounds__(kPlaneThreads) k_sweep_planes(const PlaneJob* 
 
 // ------------------------------------------------------- any line length
 
-// Reference rule for a whole line held at s[m * st], sequentially (lines
-// longer than the shared-memory tiles).
-__device__ __forceinline__ void solve_line(float* s, size_t st, const LineRule& r, const float* __restrict__ t)
+// Lines too long for a tensor box (and any line without a tensor map): one
+// warp per line, kLongLines lines per CTA (8 adjacent columns: one 32-byte
+// sector per row).  Both recurrences are affine, d_i = g_i d_{i-1} + h_i and
+// x_i = g_i x_{i+1} + d_i, so lane l takes K consecutive positions, runs
+// them from zero, the 32 (product of g, end value) pairs are scanned with
+// shuffles, and the lane runs its positions again from the value the scan
+// gives it: 4 K + 10 dependent steps where one thread per line has 2 n.
+// Values and tables are staged in shared memory with one pad per K
+// positions, so that the lanes' runs hit different banks, and a line's g
+// and values stay in registers between the passes.  A line longer than one
+// segment of 32 K positions keeps d in place in global memory between a
+// forward and a backward walk over its segments.
+//
+// What bounds it: the latency of those steps and of one round trip to
+// memory.  A diffusion step (x and y) of 701 x 530 voxels, two substrates,
+// takes 16.4 us, where one thread per line in place (n dependent,
+// uncoalesced accesses) took 516; the x sweep of 300-voxel lines (2 x 300 x
+// 300 x 60) 95 us, where 32-line tiles with bulk row copies took 335.
+template <int K>
+__host__ __device__ constexpr int long_stride() { return 32 * (K + 1) + 4; }   // 4 mod 32: 8 columns hit 8 bank groups
+
+template <int K>
+__device__ __forceinline__ int long_at(int i) { return i + i / K; }
+
+// One direction of a line's segment: v[k] = h (forward) or d (backward) in,
+// the recurrence's values out; 'edge' enters at the segment's first
+// position in walking order.  Returns the value at the last one.
+template <int K, bool BACK>
+__device__ __forceinline__ float long_scan(float (&v)[K], const float (&g)[K], float edge, int lane)
 {
-    const int n = static_cast<int>(r.n);
-    if (n >= 3) {
-        float d = 0.f;
-        for (int i = 1; i <= n - 2; ++i) {
-            const float f = (i == 1 || i == n - 2) ? r.fold : 0.f;
-            d = fmaf(__ldg(t + ((i >> 2) << 3) + (i & 3)), d, (s[i * st] + f) * __ldg(t + ((i >> 2) << 3) + 4 + (i & 3)));
-            s[i * st] = d;
-        }
-        float x = 0.f;
-        for (int i = n - 2; i >= 1; --i) {
-            x = fmaf(__ldg(t + ((i >> 2) << 3) + (i & 3)), x, s[i * st]);
-            s[i * st] = x;
+    float D = 0.f, G = 1.f;
+#pragma unroll
+    for (int q = 0; q < K; ++q) {
+        const int k = BACK ? K - 1 - q : q;
+        D = fmaf(g[k], D, v[k]);
+        G *= g[k];
+    }
+    // inclusive scan of the affine maps in walking order
+    const int pos = BACK ? 31 - lane : lane;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const float Dp = BACK ? __shfl_down_sync(0xffffffffu, D, o) : __shfl_up_sync(0xffffffffu, D, o);
+        const float Gp = BACK ? __shfl_down_sync(0xffffffffu, G, o) : __shfl_up_sync(0xffffffffu, G, o);
+        if (pos >= o) {
+            D = fmaf(G, Dp, D);
+            G *= Gp;
         }
     }
-    if (r.dir) {
-        s[0] = r.T;
-        s[(n - 1) * st] = r.T;
+    const float Dx = BACK ? __shfl_down_sync(0xffffffffu, D, 1) : __shfl_up_sync(0xffffffffu, D, 1);
+    const float Gx = BACK ? __shfl_down_sync(0xffffffffu, G, 1) : __shfl_up_sync(0xffffffffu, G, 1);
+    float x = pos == 0 ? edge : fmaf(Gx, edge, Dx);
+#pragma unroll
+    for (int q = 0; q < K; ++q) {
+        const int k = BACK ? K - 1 - q : q;
+        x = fmaf(g[k], x, v[k]);
+        v[k] = x;
     }
+    return __shfl_sync(0xffffffffu, x, BACK ? 0 : 31);
 }
 
-__global__ void __launch_bounds__(128) k_sweep_global(float* __restrict__ dens, const SweepTile* __restrict__ tiles,
-                                                      uint32_t ntiles,
-                                                      const float* __restrict__ tab, int apply_faces,
-                                                      const uint8_t* __restrict__ mask)
+template <int K>
+__global__ void __launch_bounds__(32 * kLongLines) k_sweep_long(float* __restrict__ dens,
+                                                                const SweepTile* __restrict__ tiles,
+                                                                const float* __restrict__ tab, int apply_faces,
+                                                                const uint8_t* __restrict__ mask)
 {
-    const int lane = threadIdx.x & 31;
-    const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const uint32_t nw = (gridDim.x * blockDim.x) >> 5;
-    for (uint32_t t = gw; t < ntiles; t += nw) {
-        const SweepTile tile = tiles[t];
-        if (static_cast<uint32_t>(lane) >= tile.count) continue;
-        const LineRule r = rule_of(tile);
-        if (!tile_on(r, mask)) continue;
-        const bool rows = (tile.face & TILE_ROWS) != 0;
-        // row tiles: lines tile.rs apart, unit stride; column tiles: adjacent lines, stride tile.rs
-        float* g = dens + tile.base + (rows ? static_cast<size_t>(lane) * tile.rs : static_cast<size_t>(lane));
-        const size_t st = rows ? 1 : tile.rs;
-        if (!rows && apply_faces && (tile.face & TILE_FACE) && on_face(tile, lane)) {
-            for (uint32_t j = 0; j < r.n; ++j) g[j * st] = r.T;
-        } else {
-            solve_line(g, st, r, tab + r.tab);
+    constexpr int kSeg = 32 * K, kStride = long_stride<K>();
+    extern __shared__ float sh[];
+    float* sg = sh + kLongLines * kStride;   // g of the segment's positions
+    float* si = sg + kStride;                // 1 / den
+    const SweepTile tile = tiles[blockIdx.x];
+    const LineRule r = rule_of(tile);
+    if (!tile_on(r, mask)) return;   // the whole CTA leaves together
+    const int n = static_cast<int>(r.n), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const bool rows = (tile.face & TILE_ROWS) != 0;
+    const float* t = tab + r.tab;
+    // the line and position a thread moves at step i: rows, one line per
+    // warp; columns, 8 adjacent lines per row of threads
+    const int line = rows ? warp : static_cast<int>(threadIdx.x & 7u);
+    const int p0 = rows ? lane : static_cast<int>(threadIdx.x >> 3), dp = 32;
+    const bool mine = line < static_cast<int>(tile.count);
+    const size_t ls = rows ? tile.rs : 1, ps = rows ? 1 : tile.rs;
+    float* gl = dens + tile.base + static_cast<size_t>(line) * ls;
+    float* sl = sh + line * kStride;
+    const bool face = !rows && apply_faces && (tile.face & TILE_FACE) && mine && on_face(tile, line);
+    const float* sv = sh + warp * kStride + lane * (K + 1);
+    float* sw = sh + warp * kStride + lane * (K + 1);
+    float v[K], g[K];
+
+    auto load = [&](int s0) {   // the segment's values and table; end nodes and places past the line as zeros
+        for (int p = static_cast<int>(threadIdx.x); p < kSeg; p += static_cast<int>(blockDim.x)) {
+            const int i = s0 + p;
+            sg[long_at<K>(p)] = i < n ? __ldg(t + ((i >> 2) << 3) + (i & 3)) : 0.f;
+            si[long_at<K>(p)] = i < n ? __ldg(t + ((i >> 2) << 3) + 4 + (i & 3)) : 0.f;
         }
+#pragma unroll 8
+        for (int p = p0; p < kSeg; p += dp) {
+            const int i = s0 + p;
+            sl[long_at<K>(p)] = (mine && i > 0 && i < n - 1) ? gl[static_cast<size_t>(i) * ps] : 0.f;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            v[k] = sv[k];
+            g[k] = sg[lane * (K + 1) + k];
+        }
+    };
+    auto to_rhs = [&](int s0) {   // h_i = (rho_i + fold_i) / den_i
+#pragma unroll
+        for (int k = 0; k < K; ++k) {
+            const int i = s0 + lane * K + k;
+            const float f = (i == 1 || i == n - 2) ? r.fold : 0.f;
+            v[k] = (v[k] + f) * si[lane * (K + 1) + k];
+        }
+    };
+    auto store = [&](int s0, bool last) {   // interior values (and, at the end, the end nodes' targets and the faces)
+#pragma unroll
+        for (int k = 0; k < K; ++k) sw[k] = v[k];
+        __syncthreads();
+        if (mine) {
+#pragma unroll 8
+            for (int p = p0; p < kSeg; p += dp) {
+                const int i = s0 + p;
+                if (i >= n) continue;
+                const bool end = i == 0 || i == n - 1;
+                if (last && (face || (end && r.dir))) gl[static_cast<size_t>(i) * ps] = r.T;
+                else if (!end) gl[static_cast<size_t>(i) * ps] = sl[long_at<K>(p)];
+            }
+        }
+        __syncthreads();   // the stage may be loaded again
+    };
+
+    if (n <= kSeg) {
+        load(0);
+        to_rhs(0);
+        long_scan<K, false>(v, g, 0.f, lane);
+        long_scan<K, true>(v, g, 0.f, lane);
+        store(0, true);
+        return;
+    }
+    float edge = 0.f;
+    int s0 = 0;
+    for (; s0 < n; s0 += kSeg) {
+        load(s0);
+        to_rhs(s0);
+        edge = long_scan<K, false>(v, g, edge, lane);
+        store(s0, false);
+    }
+    edge = 0.f;
+    for (s0 -= kSeg; s0 >= 0; s0 -= kSeg) {
+        load(s0);
+        edge = long_scan<K, true>(v, g, edge, lane);
+        store(s0, true);
     }
 }
 
@@ -935,7 +903,7 @@ int sweep_tma_occupancy(bool rows, int warps, int nstages, int stage_floats)
     return b;
 }
 
-cudaError_t launch_sweep_tma(cudaStream_t st, bool rows, float* dens, const SweepTile* tiles, uint32_t ntiles,
+cudaError_t launch_sweep_tma(cudaStream_t st, bool rows, const SweepTile* tiles, uint32_t ntiles,
                              const float* tab, const void* tmaps, int apply_faces,
                              const uint8_t* mask, unsigned* status, TmaCfg cfg)
 {
@@ -945,11 +913,11 @@ cudaError_t launch_sweep_tma(cudaStream_t st, bool rows, float* dens, const Swee
         return cudaErrorInvalidValue;
     const size_t smem = sweep_tma_smem(cfg.warps, cfg.stages, cfg.stage_floats);
     if (rows)
-        k_sweep_tma<true><<<cfg.grid, cfg.warps * 32, smem, st>>>(dens, tiles, ntiles, tab, tmaps,
+        k_sweep_tma<true><<<cfg.grid, cfg.warps * 32, smem, st>>>(tiles, ntiles, tab, tmaps,
                                                                    cfg.stage_floats, cfg.stages, cfg.tab_floats,
                                                                    apply_faces, mask, status);
     else
-        k_sweep_tma<false><<<cfg.grid, cfg.warps * 32, smem, st>>>(dens, tiles, ntiles, tab, tmaps,
+        k_sweep_tma<false><<<cfg.grid, cfg.warps * 32, smem, st>>>(tiles, ntiles, tab, tmaps,
                                                                     cfg.stage_floats, cfg.stages, cfg.tab_floats,
                                                                     apply_faces, mask, status);
     return cudaGetLastError();
@@ -1086,13 +1054,26 @@ cudaError_t launch_sweep_planes(cudaStream_t st, const PlaneJob* jobs, uint32_t 
     return cudaGetLastError();
 }
 
-cudaError_t launch_sweep_global(cudaStream_t st, float* dens, const SweepTile* tiles, uint32_t ntiles,
-                                const float* tab, int apply_faces, const uint8_t* mask,
-                                int grid)
+template <int K>
+static cudaError_t long_variant(cudaStream_t st, float* dens, const SweepTile* tiles, uint32_t ntiles, const float* tab,
+                                int apply_faces, const uint8_t* mask)
+{
+    const size_t smem = static_cast<size_t>(kLongLines + 2) * long_stride<K>() * sizeof(float);   // at most 43 KB
+    k_sweep_long<K><<<ntiles, 32 * kLongLines, smem, st>>>(dens, tiles, tab, apply_faces, mask);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_sweep_long(cudaStream_t st, float* dens, const SweepTile* tiles, uint32_t ntiles, const float* tab,
+                              int nmax, int apply_faces, const uint8_t* mask)
 {
     if (ntiles == 0) return cudaSuccess;
-    k_sweep_global<<<grid, 128, 0, st>>>(dens, tiles, ntiles, tab, apply_faces, mask);
-    return cudaGetLastError();
+    // positions per lane: the fewest that hold the longest line in one
+    // segment (a lane's steps, registers and shared memory grow with them),
+    // at most 32; longer lines take several segments
+    if (nmax <= 32 * 12) return long_variant<12>(st, dens, tiles, ntiles, tab, apply_faces, mask);
+    if (nmax <= 32 * 16) return long_variant<16>(st, dens, tiles, ntiles, tab, apply_faces, mask);
+    if (nmax <= 32 * 24) return long_variant<24>(st, dens, tiles, ntiles, tab, apply_faces, mask);
+    return long_variant<32>(st, dens, tiles, ntiles, tab, apply_faces, mask);
 }
 
 cudaError_t launch_dirichlet(cudaStream_t st, float* dens, const FaceJob* jobs, uint32_t njobs)

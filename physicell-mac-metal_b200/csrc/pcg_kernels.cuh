@@ -52,8 +52,9 @@ __host__ __device__ constexpr uint32_t tab_floats(uint32_t n) { return ((n + 3u)
 // (the row pitch) apart.  Column tiles (y and z sweeps): 'nslab' adjacent
 // slabs (outer coordinates outer .. outer + nslab - 1) of 'count' (<= width)
 // adjacent columns from x = i0, width * nslab <= 32; lane = slab * width +
-// column.  Without a tensor map a column tile has width 32 and one slab, and
-// its lines start at 'base' with element stride 'rs'.
+// column.  Tiles without TILE_TENSOR (k_sweep_long) hold up to kLongLines
+// lines: rows as above, columns of one slab (width kLongLines) starting at
+// 'base' with element stride 'rs'.
 struct SweepTile {
     uint64_t base;
     uint32_t count;
@@ -93,7 +94,7 @@ __host__ __device__ constexpr uint32_t row_smem_pitch(uint32_t n) { return (((n 
 constexpr uint32_t kRowTensorMaxN = 252;
 
 // Device status word bits (a kernel that cannot finish records why and returns).
-enum : unsigned { PCG_DEV_TIMEOUT = 1u, PCG_DEV_ALIGN = 2u };
+enum : unsigned { PCG_DEV_TIMEOUT = 1u };
 // Test switches, in the word after the status word: PCG_DEV_TEST_GIVE_UP
 // makes the first wait of every plane CTA report that its bound ran out at
 // once (the wait for the CTA's own copies before it exits keeps its bound).
@@ -175,14 +176,13 @@ __host__ __device__ constexpr uint32_t plane_floats(uint32_t nx, uint32_t ny, bo
 
 struct TmaCfg { int warps; int stages; int stage_floats; int grid; int tab_floats; };
 
-// Longest line staged in shared memory; longer lines take the one-thread-
-// per-line kernel.  Tables are the chunked LineRule tables (float).
-constexpr uint32_t kTmaMaxN = 512;
+// Lines per CTA of the kernel for lines without a tensor map (one warp each).
+constexpr uint32_t kLongLines = 8;
 
 size_t sweep_tma_smem(int warps, int nstages, int stage_floats);
 int sweep_tma_occupancy(bool rows, int warps, int nstages, int stage_floats);   // CTAs per SM (0 = does not fit)
-// tmaps: one 128-byte CUtensorMap per rule (64-byte aligned, global memory)
-// for the tiles flagged TILE_TENSOR; may be null otherwise.
+// tmaps: the 128-byte CUtensorMaps the tiles name (64-byte aligned, global
+// memory); every tile is flagged TILE_TENSOR.
 // Fused x + y sweeps, one CTA per plane; 'floats' = the largest
 // plane_floats of the jobs.
 cudaError_t launch_sweep_planes(cudaStream_t st, const PlaneJob* jobs, uint32_t njobs, const float* tab,
@@ -198,7 +198,7 @@ size_t sweep_planes_smem(uint32_t floats);
 int sweep_planes_ctas(uint32_t floats);
 bool encode_plane_map(void* map128, float* block, uint32_t nx, uint32_t ny, uint64_t rows, uint32_t px);
 bool encode_xz_plane_map(void* map128, float* block, uint32_t nx, uint32_t ny, uint32_t nz, uint32_t px);
-cudaError_t launch_sweep_tma(cudaStream_t st, bool rows, float* dens, const SweepTile* tiles, uint32_t ntiles,
+cudaError_t launch_sweep_tma(cudaStream_t st, bool rows, const SweepTile* tiles, uint32_t ntiles,
                              const float* tab, const void* tmaps, int apply_faces,
                              const uint8_t* mask, unsigned* status, TmaCfg cfg);
 // Encode the 3-D tensor map of one substrate block (rows px floats apart)
@@ -211,10 +211,10 @@ bool encode_column_map(void* map128, float* block, uint32_t nx, uint32_t ny, uin
 // Encode the 2-D tensor map of one substrate block seen as rows x nx (rows
 // px floats apart) with a box of row_smem_pitch(nx) x 32 (x tiles).
 bool encode_row_map(void* map128, float* block, uint32_t nx, uint64_t rows, uint32_t px);
-// Any line length: one thread per line, d kept in place in global memory.
-cudaError_t launch_sweep_global(cudaStream_t st, float* dens, const SweepTile* tiles, uint32_t ntiles,
-                                const float* tab, int apply_faces, const uint8_t* mask,
-                                int grid);
+// Any line length, one warp per line, one CTA per tile of up to kLongLines
+// lines; nmax = the longest line of the tiles.
+cudaError_t launch_sweep_long(cudaStream_t st, float* dens, const SweepTile* tiles, uint32_t ntiles, const float* tab,
+                              int nmax, int apply_faces, const uint8_t* mask);
 
 // applyDirichletBC over instances [0, n_inst): faces of Dirichlet substrates.
 struct FaceJob { uint64_t base; uint32_t nx, ny, nz, px; float T; uint32_t _pad; };

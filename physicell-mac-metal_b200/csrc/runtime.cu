@@ -654,14 +654,14 @@ static void fill_rule(SweepTile& t, const LineRule& r)
     t.inst = r.inst | (r.dir ? 0x80000000u : 0u);
 }
 
-// Tile lists of one axis: lines up to kTmaMaxN go to the pipelined TMA
-// kernels (x: 32 lines per tile; y/z: 32 columns per tile), longer lines to
-// the one-thread-per-line kernel.
+// Tile lists of one axis: lines with a tensor map (up to 252 / 256
+// positions) go to the pipelined TMA kernels (x: 32 lines per tile; y/z: 32
+// columns per tile), the others to the one-warp-per-line kernel.
 int Diffusion::build_axis(int axis, const std::vector<uint8_t>* skip, std::vector<SweepList>& ls)
 {
-    std::vector<SweepTile> fast_t, glob_t;
-    int fast_nmax = 0, glob_nmax = 0;
-    uint64_t fast_lines = 0, glob_lines = 0, fast_units = 0, glob_units = 0;
+    std::vector<SweepTile> fast_t, long_t;
+    int fast_nmax = 0, long_nmax = 0;
+    uint64_t fast_lines = 0, long_lines = 0, fast_units = 0, long_units = 0;
     const int kind_fast = axis == 0 ? 0 : 1;
     for (size_t i = 0; i < inst.size(); ++i) {
         if (skip && (*skip)[i]) continue;
@@ -670,31 +670,33 @@ int Diffusion::build_axis(int axis, const std::vector<uint8_t>* skip, std::vecto
         const int nd = d.ndim();
         if (axis == 2 && nd < 3) continue;
         const uint32_t n = axis_n(g, axis);
-        const bool fast = n <= kTmaMaxN;
-        auto& out = fast ? fast_t : glob_t;
-        int& nmax = fast ? fast_nmax : glob_nmax;
-        uint64_t& nl = fast ? fast_lines : glob_lines;
-        (fast ? fast_units : glob_units) += d.nvox() * g.n_substrates;
-        nmax = std::max<int>(nmax, static_cast<int>(n));
         const bool final_axis = axis == nd - 1;
         for (uint32_t s = 0; s < g.n_substrates; ++s) {
             const uint32_t rule = rule_of(i, s, axis);
             const bool dir = d.subs[s].dirichlet_enabled != 0;
             const uint64_t sbase = d.dens_off + s * d.pitch;
+            // column maps of every width (bits 0-2), the x rules' row map in bit 0
+            const bool fast = axis == 0 ? (tensor_ok_[rule] & 1u) != 0 : tensor_ok_[rule] == 7u;
+            auto& out = fast ? fast_t : long_t;
+            int& nmax = fast ? fast_nmax : long_nmax;
+            uint64_t& nl = fast ? fast_lines : long_lines;
+            (fast ? fast_units : long_units) += d.nvox();
+            nmax = std::max<int>(nmax, static_cast<int>(n));
             if (axis == 0) {
                 const uint64_t lines = d.rows();
-                for (uint64_t l0 = 0; l0 < lines; l0 += 32) {
+                const uint64_t per = fast ? 32 : kLongLines;
+                for (uint64_t l0 = 0; l0 < lines; l0 += per) {
                     SweepTile t{};
                     t.base = sbase + l0 * d.px;
                     fill_rule(t, h_rules_[rule]);
-                    t.count = static_cast<uint32_t>(std::min<uint64_t>(32, lines - l0));
+                    t.count = static_cast<uint32_t>(std::min<uint64_t>(per, lines - l0));
                     t.rs = d.px;
                     t.nx = g.nx;
                     t.outer = static_cast<uint32_t>(l0);
                     t.map = rule * kMapsPerRule;
                     t.width = 32;
                     t.nslab = 1;
-                    t.face = TILE_ROWS | ((fast && tensor_ok_[rule]) ? TILE_TENSOR : 0u);
+                    t.face = TILE_ROWS | (fast ? TILE_TENSOR : 0u);
                     out.push_back(t);
                 }
                 nl += lines;
@@ -706,18 +708,12 @@ int Diffusion::build_axis(int axis, const std::vector<uint8_t>* skip, std::vecto
                 const uint32_t outer = axis == 1 ? g.nz : g.ny;
                 const uint64_t ostride = axis == 1 ? static_cast<uint64_t>(d.px) * g.ny : d.px;
                 const uint32_t rs = axis == 1 ? d.px : d.px * g.ny;
-                for (uint32_t i0 = 0; i0 < g.nx; i0 += 32) {
-                    const uint32_t cnt = std::min<uint32_t>(32, g.nx - i0);
-                    int w = 0;
-                    if (fast && tensor_ok_[rule]) {
-                        if (cnt <= 8 && (tensor_ok_[rule] & 4u)) w = 2;
-                        else if (cnt <= 16 && (tensor_ok_[rule] & 2u)) w = 1;
-                        if (!(tensor_ok_[rule] & (1u << w))) w = -1;
-                    } else {
-                        w = -1;
-                    }
-                    const uint32_t width = w < 0 ? 32u : (32u >> w);
-                    const uint32_t group = 32u / width;
+                const uint32_t per = fast ? 32u : kLongLines;
+                for (uint32_t i0 = 0; i0 < g.nx; i0 += per) {
+                    const uint32_t cnt = std::min<uint32_t>(per, g.nx - i0);
+                    const int w = !fast || cnt > 16 ? 0 : cnt > 8 ? 1 : 2;
+                    const uint32_t width = fast ? 32u >> w : kLongLines;
+                    const uint32_t group = fast ? 32u / width : 1u;
                     for (uint32_t o = 0; o < outer; o += group) {
                         SweepTile t{};
                         t.base = sbase + o * ostride + i0;
@@ -730,8 +726,8 @@ int Diffusion::build_axis(int axis, const std::vector<uint8_t>* skip, std::vecto
                         t.outer_n = outer;
                         t.width = static_cast<uint16_t>(width);
                         t.nslab = static_cast<uint16_t>(std::min(group, outer - o));
-                        t.map = rule * kMapsPerRule + static_cast<uint32_t>(w < 0 ? 0 : w);
-                        if (w >= 0) t.face |= TILE_TENSOR;
+                        t.map = rule * kMapsPerRule + static_cast<uint32_t>(w);
+                        if (fast) t.face |= TILE_TENSOR;
                         if (axis == 2) t.face |= TILE_AXIS_Z;
                         if (final_axis && dir) t.face |= TILE_FACE;
                         out.push_back(t);
@@ -744,7 +740,7 @@ int Diffusion::build_axis(int axis, const std::vector<uint8_t>* skip, std::vecto
     // larger lines first so the persistent loop ends evenly
     auto by_n = [](const SweepTile& a, const SweepTile& b) { return a.n > b.n; };
     std::stable_sort(fast_t.begin(), fast_t.end(), by_n);
-    std::stable_sort(glob_t.begin(), glob_t.end(), by_n);
+    std::stable_sort(long_t.begin(), long_t.end(), by_n);
     ls.clear();
     ls.resize(2);
     ls[0].kind = kind_fast;
@@ -753,12 +749,12 @@ int Diffusion::build_axis(int axis, const std::vector<uint8_t>* skip, std::vecto
     ls[0].lines = fast_lines;
     ls[0].units = fast_units;
     ls[1].kind = 2;
-    ls[1].nmax = glob_nmax;
-    ls[1].n = static_cast<uint32_t>(glob_t.size());
-    ls[1].lines = glob_lines;
-    ls[1].units = glob_units;
+    ls[1].nmax = long_nmax;
+    ls[1].n = static_cast<uint32_t>(long_t.size());
+    ls[1].lines = long_lines;
+    ls[1].units = long_units;
     for (int q = 0; q < 2; ++q) {
-        const auto& v = q == 0 ? fast_t : glob_t;
+        const auto& v = q == 0 ? fast_t : long_t;
         PCG_CU(ctx, ls[q].tiles.alloc(std::max<size_t>(v.size(), 1) * sizeof(SweepTile)));
         if (!v.empty())
             PCG_CU(ctx, cudaMemcpyAsync(ls[q].tiles.p, v.data(), v.size() * sizeof(SweepTile), cudaMemcpyHostToDevice, ctx->stream));
@@ -785,12 +781,7 @@ static int tma_stage_floats(const SweepList& l)
 
 int Diffusion::config_list(SweepList& l, int param)
 {
-    if (l.n == 0) return PCG_OK;
-    if (l.kind == 2) {
-        const uint64_t ctas = (static_cast<uint64_t>(l.n) * 32 + 127) / 128;
-        l.ggrid = static_cast<int>(std::min<uint64_t>(std::max<uint64_t>(ctas, 1), static_cast<uint64_t>(ctx->sms) * 16));
-        return PCG_OK;
-    }
+    if (l.n == 0 || l.kind == 2) return PCG_OK;   // kind 2: one CTA per tile, nothing to choose
     const bool rows = l.kind == 0;
     const int sf = tma_stage_floats(l);
     int best_w = 0, best_s = 0, best_occ = 0;
@@ -847,9 +838,9 @@ int Diffusion::launch_list(const SweepList& l, bool fuse, const uint8_t* mask)
     const SweepTile* t = l.tiles.as<SweepTile>();
     const float* tb = tab.as<float>();
     cudaError_t e;
-    if (l.kind == 2) e = launch_sweep_global(ctx->stream, d, t, l.n, tb, fuse ? 1 : 0, mask, l.ggrid);
+    if (l.kind == 2) e = launch_sweep_long(ctx->stream, d, t, l.n, tb, l.nmax, fuse ? 1 : 0, mask);
     else
-        e = launch_sweep_tma(ctx->stream, l.kind == 0, d, t, l.n, tb, tmaps.p, fuse ? 1 : 0, mask, ctx->status, l.tc);
+        e = launch_sweep_tma(ctx->stream, l.kind == 0, t, l.n, tb, tmaps.p, fuse ? 1 : 0, mask, ctx->status, l.tc);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "sweep launch");
     ctx->launches++;
     return PCG_OK;
@@ -1058,7 +1049,7 @@ std::string Diffusion::describe() const
             if (l.kind != 2)
                 o << (l.kind == 0 ? "x-tma(" : "cols-tma(") << "warps=" << l.tc.warps << ",stages=" << l.tc.stages
                   << ",grid=" << l.tc.grid;
-            else o << "global(grid=" << l.ggrid;
+            else o << "warp-lines(";
             o << ",tiles=" << l.n << ",nmax=" << l.nmax << ") ";
         }
     return o.str();

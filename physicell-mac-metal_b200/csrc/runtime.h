@@ -171,12 +171,11 @@ struct PlaneList {
 };
 
 struct SweepList {
-    int kind = 0;              // 0 row tiles (TMA), 1 column tiles (TMA), 2 any length (global)
+    int kind = 0;              // 0 row tiles (TMA), 1 column tiles (TMA), 2 any length (one warp per line)
     int nmax = 0;
     uint32_t n = 0;
     DevBuf tiles;
     TmaCfg tc{4, 3, 0, 1};
-    int ggrid = 1;
     uint64_t lines = 0;        // lines covered (for tuning keys)
     uint64_t units = 0;        // voxel-substrates covered
 };
