@@ -167,7 +167,7 @@ int Batch::create(pcg_ctx* c, const pcg_instance_desc* descs, uint32_t n, const 
     }
     c_.inst_dirty = true;
     PCG_TRY(c_.sync_inst());
-    PCG_TRY(m_.create(ctx, moff, cell_cap));
+    PCG_TRY(m_.create(ctx, moff, cell_cap, n));
     m_.lazy_sorder = true;   // only pcg_batch_mech_bins reads the stable order
     PCG_CU(ctx, cudaStreamSynchronize(ctx->stream));
     if (c_.n) PCG_TRY(c_.prepare_secretion(dt_diff, d.total_vox));

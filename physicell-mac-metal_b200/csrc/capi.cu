@@ -567,7 +567,7 @@ pcg_status pcg_mech_create(pcg_ctx* ctx, const pcg_mechanics_params* p, float x_
     m->oy = y_min;
     m->oz = z_min;
     const uint32_t V = p->mech_grid_nx * p->mech_grid_ny * p->mech_grid_nz;
-    int rc = m->m.create(ctx, V, max_cells);
+    int rc = m->m.create(ctx, V, max_cells, 1);
     if (rc != PCG_OK) {
         delete m;
         return rc;

@@ -252,14 +252,16 @@ cudaError_t launch_secrete(cudaStream_t st, float* dens, const uint32_t* run_sta
 // the stable order (sorder: cells by voxel, ascending index within a voxel;
 // skipped when null) and, in the force order (by voxel, then x, index
 // breaking ties), the positions / radii (spos) and the strengths (sprm:
-// sqrt repulsion, sqrt adhesion, the cell's index as bits, 1 / relmax).
+// sqrt repulsion, sqrt adhesion, the cell's index as bits, 1 / relmax), and
+// per instance the largest radius (reach: zeroed words, bits of a float).
 // launch_mech_stable_order writes sorder alone from the same binning.
 cudaError_t launch_mech_bin(cudaStream_t st, float* soa, uint32_t stride, uint32_t n,
                             const uint32_t* cell_inst, const CellInst* insts,
                             uint32_t* keys, uint32_t* slots, uint32_t* counts, const uint8_t* mask, int block = 256);
 cudaError_t launch_mech_order(cudaStream_t st, const float* soa, uint32_t stride, const uint32_t* keys,
                               const uint32_t* slots, const uint32_t* start, uint32_t n, uint2* placed,
-                              uint32_t* sorder, float4* spos, float4* sprm, int block = 256);
+                              const uint32_t* cell_inst, uint32_t* reach, uint32_t* sorder, float4* spos,
+                              float4* sprm, int block = 256);
 cudaError_t launch_mech_stable_order(cudaStream_t st, const uint32_t* keys, const uint32_t* start,
                                      const uint2* placed, uint32_t n, uint32_t* sorder);
 // Launch shape of the force pass: threads per block (a multiple of 32, at
@@ -275,8 +277,9 @@ struct ForceShape {
 cudaError_t mech_forces_prepare();
 cudaError_t launch_mech_forces(cudaStream_t st, const float4* spos, const float4* sprm,
                                const uint32_t* start, uint32_t n,
-                               const uint32_t* cell_inst, const CellInst* insts, float* soa, uint32_t stride,
-                               uint32_t* diag_cnt, uint32_t* diag_hash, const uint8_t* mask, ForceShape shape);
+                               const uint32_t* cell_inst, const CellInst* insts, const uint32_t* reach, float* soa,
+                               uint32_t stride, uint32_t* diag_cnt, uint32_t* diag_hash, const uint8_t* mask,
+                               ForceShape shape);
 // Copies of a removal plan: (dst, src) pairs, each cell's 28 SoA fields,
 // 4 x S rates (arrays of rate_cap doubles, [cell * S + s]), active flag and
 // three FP64 master positions (arrays of stride doubles; pos64 may be null).

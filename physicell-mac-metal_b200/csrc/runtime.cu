@@ -1439,7 +1439,7 @@ uint64_t Cells::device_bytes() const
 
 // ------------------------------------------------------------------ mechanics
 
-int Mechanics::create(pcg_ctx* c, uint32_t tmv, uint32_t maxc)
+int Mechanics::create(pcg_ctx* c, uint32_t tmv, uint32_t maxc, uint32_t n_instances)
 {
     ctx = c;
     total_mvox = tmv;
@@ -1448,7 +1448,7 @@ int Mechanics::create(pcg_ctx* c, uint32_t tmv, uint32_t maxc)
     for (DevBuf* b : {&keys, &slots, &sorder, &dcnt, &dhash})
         PCG_CU(ctx, b->alloc(static_cast<size_t>(cap) * sizeof(uint32_t)));
     PCG_CU(ctx, placed.alloc(static_cast<size_t>(cap) * sizeof(uint2)));
-    PCG_CU(ctx, counts.alloc((static_cast<size_t>(tmv) + 1) * sizeof(uint32_t)));
+    PCG_CU(ctx, counts.alloc((static_cast<size_t>(tmv) + 1 + n_instances) * sizeof(uint32_t)));
     PCG_CU(ctx, start.alloc((static_cast<size_t>(tmv) + 1) * sizeof(uint32_t)));
     PCG_CU(ctx, cudaMemsetAsync(start.p, 0, start.bytes, ctx->stream));
     PCG_CU(ctx, scan_scr.alloc(scan_scratch_bytes(static_cast<uint64_t>(tmv) + 1)));
@@ -1485,8 +1485,8 @@ int Mechanics::binsort(Cells& c, const uint8_t* mask)
     e = scan_exclusive(st, counts.as<uint32_t>(), start.as<uint32_t>(), static_cast<uint64_t>(total_mvox) + 1, scan_scr.p);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "start-table scan");
     e = launch_mech_order(st, c.soa.as<float>(), c.max_cells, keys.as<uint32_t>(), slots.as<uint32_t>(),
-                          start.as<uint32_t>(), c.n, placed.as<uint2>(), lazy_sorder ? nullptr : sorder.as<uint32_t>(),
-                          spos.as<float4>(), sprm.as<float4>(), bin_block);
+                          start.as<uint32_t>(), c.n, placed.as<uint2>(), c.cell_inst.as<uint32_t>(), reach(),
+                          lazy_sorder ? nullptr : sorder.as<uint32_t>(), spos.as<float4>(), sprm.as<float4>(), bin_block);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "bin order launch");
     ctx->launches += launches_forces(c.n) - 2;   // the memset is not a kernel; forces counted below
     sorder_valid = !lazy_sorder;
@@ -1509,7 +1509,7 @@ int Mechanics::force_pass(Cells& c, const uint8_t* mask)
     if (c.n == 0) return PCG_OK;
     cudaStream_t st = ctx->stream;
     cudaError_t e = launch_mech_forces(st, spos.as<float4>(), sprm.as<float4>(), start.as<uint32_t>(), c.n,
-                           c.cell_inst.as<uint32_t>(), c.inst.as<CellInst>(), c.soa.as<float>(), c.max_cells, diag ? dcnt.as<uint32_t>() : nullptr, diag ? dhash.as<uint32_t>() : nullptr,
+                           c.cell_inst.as<uint32_t>(), c.inst.as<CellInst>(), reach(), c.soa.as<float>(), c.max_cells, diag ? dcnt.as<uint32_t>() : nullptr, diag ? dhash.as<uint32_t>() : nullptr,
                            mask, fshape);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "forces launch");
     ctx->launches++;

@@ -328,19 +328,20 @@ public:
     // sorder_valid: it matches the last binning.
     bool lazy_sorder = false, sorder_valid = false;
     // binning: keys / slots (voxel key and arrival slot per cell), counts
-    // (per voxel, + 1), start (the cell-start table), placed ((x key, cell)
+    // (per voxel, + 1, then a word per instance: its largest radius, reach()), start (the cell-start table), placed ((x key, cell)
     // in arrival order per voxel), sorder (the stable order: by voxel, then
     // index), spos / sprm (positions and strengths in the force order: by
     // voxel, then x; the cell's index in sprm's third component)
     DevBuf keys, slots, placed, sorder, counts, start, scan_scr, spos, sprm, dcnt, dhash;
 
-    int create(pcg_ctx* c, uint32_t total_mvox, uint32_t max_cells);
+    int create(pcg_ctx* c, uint32_t total_mvox, uint32_t max_cells, uint32_t n_instances);
     int forces(Cells& c, const uint8_t* mask);       // binsort + force_pass
     int binsort(Cells& c, const uint8_t* mask);      // bin, counting sort, cell-start table, sorted SoA
     int stable_order(uint32_t n);                    // sorder from the last binning, when not yet made
     int force_pass(Cells& c, const uint8_t* mask);
     int integrate(Cells& c, float dt_override, const uint8_t* mask);
     int launches_forces(uint32_t n) const;
+    uint32_t* reach() const { return counts.as<uint32_t>() + total_mvox + 1; }
     uint64_t device_bytes() const;
 };
 
