@@ -12,8 +12,15 @@
 // reference's two passes are
 //     forward   d_i = g_i d_{i-1} + h_i        (d_0 = 0)
 //     backward  x_i = g_i x_{i+1} + d_i        (x_{n-1} = 0)
-// one FMUL + one FFMA, then one FFMA per value.  End nodes keep their value
-// or take the Dirichlet target.
+// one FMUL + one FFMA, then one FFMA per value, 2 n dependent steps.  Here a
+// line is eliminated from both ends towards its middle (a twisted
+// factorisation): the left half as above, the right half by the mirrored
+// recurrence (the matrix is symmetric, so its coefficients are the same
+// ones counted from the right end), a 2 x 2 system in the middle, and both
+// halves substituted outwards.  The same operations per value, but two
+// independent chains of n / 2 each way: one thread runs them side by side
+// (split_line), or two threads take one each (half_line).  End nodes keep
+// their value or take the Dirichlet target.
 //
 // Data movement.  density is [s][k][j][i] FP32 with rows padded to a pitch
 // px = nx rounded up to 4 floats, so every row starts on 16 bytes.  Each
@@ -228,10 +235,11 @@ __device__ __forceinline__ void issue_tile_store(const SweepTile& tile, const vo
 
 // ------------------------------------------------------------------ solves in shared memory
 
-// Coefficient table of one rule: line positions in chunks of 4, each chunk
-// 8 floats {g[4], inv[4]} (32-byte aligned), g_i = c / den_i, inv_i = 1 / den_i;
-// zero at the end nodes.  The tile solves read the copy staged in shared
-// memory next to the tile.
+// Coefficient table of one rule, staged in shared memory next to its lines
+// (layout: SplitTable).  A half's chunk k holds the coefficients of its 4
+// positions in the order the half is walked in, {g[4], inv[4]} (32-byte
+// aligned), g_i = c / den_i, inv_i = 1 / den_i; zero at the end node and past
+// the line.
 __device__ __forceinline__ float tab_g(const float* t, int i) { return t[((i >> 2) << 3) + (i & 3)]; }
 __device__ __forceinline__ float tab_inv(const float* t, int i) { return t[((i >> 2) << 3) + 4 + (i & 3)]; }
 __device__ __forceinline__ float4 tab_g4(const float* t, int q) { return *reinterpret_cast<const float4*>(t + (q << 3)); }
@@ -240,8 +248,7 @@ __device__ __forceinline__ float4 tab_inv4(const float* t, int q)
     return *reinterpret_cast<const float4*>(t + (q << 3) + 4);
 }
 
-// One chunk of the forward / backward pass (positions 4q..4q+3): all four,
-// or those with place u in [lo, hi] at the ends of the line.
+// One chunk of the forward / backward pass, in walking order.
 __device__ __forceinline__ float fwd1(float g, float iv, float d, float& v)
 {
     d = fmaf(g, d, v * iv);
@@ -268,106 +275,143 @@ __device__ __forceinline__ float bwd4(float4& v, float4 g, float x)
     x = bwd1(g.y, x, v.y);
     return bwd1(g.x, x, v.x);
 }
-__device__ __forceinline__ float fwd4p(float4& v, float4 g, float4 iv, float d, int lo, int hi)
+__device__ __forceinline__ float4 reversed(float4 v) { return make_float4(v.w, v.z, v.y, v.x); }
+
+// The end node of a half leaves its first chunk (with what lies before it,
+// 'lead' places past the line) and the first interior node takes the fold,
+// unless it lies in the next chunk (lead == 3).  Returns the end node.
+__device__ __forceinline__ float take_end(float4& a, int lead, float fold)
 {
-    if (lo <= 0 && 0 <= hi) d = fwd1(g.x, iv.x, d, v.x);
-    if (lo <= 1 && 1 <= hi) d = fwd1(g.y, iv.y, d, v.y);
-    if (lo <= 2 && 2 <= hi) d = fwd1(g.z, iv.z, d, v.z);
-    if (lo <= 3 && 3 <= hi) d = fwd1(g.w, iv.w, d, v.w);
-    return d;
+    const float end = lead == 0 ? a.x : lead == 1 ? a.y : lead == 2 ? a.z : a.w;
+    a.x = 0.f;
+    a.y = lead == 0 ? a.y + fold : 0.f;
+    a.z = lead == 0 ? a.z : lead == 1 ? a.z + fold : 0.f;
+    a.w = lead <= 1 ? a.w : lead == 2 ? a.w + fold : 0.f;
+    return end;
 }
-__device__ __forceinline__ float bwd4p(float4& v, float4 g, float x, int lo, int hi)
+__device__ __forceinline__ void put_end(float4& a, int lead, float end)
 {
-    if (lo <= 3 && 3 <= hi) x = bwd1(g.w, x, v.w);
-    if (lo <= 2 && 2 <= hi) x = bwd1(g.z, x, v.z);
-    if (lo <= 1 && 1 <= hi) x = bwd1(g.y, x, v.y);
-    if (lo <= 0 && 0 <= hi) x = bwd1(g.x, x, v.x);
-    return x;
+    if (lead == 0) a.x = end;
+    else if (lead == 1) a.y = end;
+    else if (lead == 2) a.z = end;
+    else a.w = end;
 }
 
-// Both passes of one line over positions 1..n-2 (n >= 3), chunk by chunk:
-// ld(q) returns chunk q (positions 4q..4q+3) from shared memory and st(q, v)
-// writes it back.  The two end chunks are peeled off, so the main loops run
-// over whole chunks with no per-position tests; each loop keeps the next
-// chunk and its coefficients loaded while the current chunk's dependent
-// FFMAs run.  Only chunks up to the one holding position n - 2 are touched;
-// places past the line's end in that chunk are written back unchanged.
+// Both halves of one line by one thread, in shared memory, over positions
+// 1..n-2 (n >= 3): ld(q) returns chunk q (positions 4q..4q+3), st(q, v)
+// writes it back; the end nodes keep their values.  The left half is the
+// first SplitTable(n).hl chunks.  Each pass takes a chunk of either half at
+// a time, the next ones loaded while the current ones' chains run.
 template <class LD, class ST>
-__device__ __forceinline__ void thomas_line(const float* t, int n, LD ld, ST st)
+__device__ __forceinline__ void split_line(const float* t, int n, float fold, LD ld, ST st)
 {
-    const int ql = (n - 2) >> 2;      // chunk of position n - 2
-    const int hl = n - 2 - 4 * ql;    // its place in that chunk
-    // forward: chunk 0 (from position 1), whole chunks 1..ql-1, chunk ql
-    float d = 0.f;
-    {
-        float4 v0 = ld(0);
-        if (ql == 0) {
-            d = fwd4p(v0, tab_g4(t, 0), tab_inv4(t, 0), d, 1, hl);
-            st(0, v0);
-        } else {
-            float4 a = ld(1), ga = tab_g4(t, 1), ia = tab_inv4(t, 1);
-            d = fwd4p(v0, tab_g4(t, 0), tab_inv4(t, 0), d, 1, 3);
-            st(0, v0);
-            int q = 1;   // a holds chunk q
-            for (; q + 1 < ql; q += 2) {
-                float4 b = ld(q + 1), gb = tab_g4(t, q + 1), ib = tab_inv4(t, q + 1);
-                d = fwd4(a, ga, ia, d);
-                st(q, a);
-                a = ld(q + 2);
-                ga = tab_g4(t, q + 2);
-                ia = tab_inv4(t, q + 2);
-                d = fwd4(b, gb, ib, d);
-                st(q + 1, b);
+    const SplitTable sp(n);
+    const int nq = sp.nq, hl = sp.hl, hr = nq - hl;
+    const float* tr = t + sp.right();
+    if (!sp.right_has_interior()) {   // n = 3, 4, 5 or 9: the left half alone
+        float4 c0 = ld(0), c1 = hl > 1 ? ld(1) : make_float4(0.f, 0.f, 0.f, 0.f);
+        float a[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+        float d = 0.f, x = 0.f;
+#pragma unroll
+        for (int i = 1; i < 8; ++i)
+            if (i <= n - 2) {
+                if (i == 1 || i == n - 2) a[i] += fold;
+                d = fwd1(tab_g(t, i), tab_inv(t, i), d, a[i]);
             }
-            if (q < ql) {   // q == ql - 1: one whole chunk, then chunk ql
-                float4 b = ld(ql), gb = tab_g4(t, ql), ib = tab_inv4(t, ql);
-                d = fwd4(a, ga, ia, d);
-                st(q, a);
-                d = fwd4p(b, gb, ib, d, 0, hl);
-                st(ql, b);
-            } else {        // a holds chunk ql
-                d = fwd4p(a, ga, ia, d, 0, hl);
-                st(ql, a);
-            }
-        }
-    }
-    // backward: chunk ql, whole chunks ql-1..1, chunk 0 (down to position 1)
-    float x = 0.f;
-    if (ql == 0) {
-        float4 w = ld(0);
-        x = bwd4p(w, tab_g4(t, 0), x, 1, hl);
-        st(0, w);
+#pragma unroll
+        for (int i = 7; i >= 1; --i)
+            if (i <= n - 2) x = bwd1(tab_g(t, i), x, a[i]);
+        st(0, make_float4(a[0], a[1], a[2], a[3]));
+        if (hl > 1) st(1, make_float4(a[4], a[5], a[6], a[7]));
         return;
     }
-    float4 a = ld(ql), ga = tab_g4(t, ql);
-    int q = ql;
-    {
-        float4 b = ld(q - 1), gb = tab_g4(t, q - 1);
-        x = bwd4p(a, ga, x, 0, hl);
-        st(q, a);
-        a = b;
-        ga = gb;
-        --q;
+    const int lead = 4 * nq - n;
+    const float fold1 = lead == 3 ? fold : 0.f;
+    const float* tj = t + sp.middle();
+    const int kc = min(__float_as_int(tj[3]), hr);   // chunks [kc, ..) of both halves: one g, one inv
+    float4 a = ld(0), b = reversed(ld(nq - 1));
+    const float4 b0 = b;
+    float4 gl = tab_g4(t, 0), il = tab_inv4(t, 0), gr = tab_g4(tr, 0), ir = tab_inv4(tr, 0);
+    const float lo = take_end(a, 0, fold);
+    take_end(b, lead, fold);
+    float dl = 0.f, dr = 0.f;
+    int k = 0;
+    for (; k < kc && k + 1 < hr; ++k) {
+        const float4 an = ld(k + 1), gln = tab_g4(t, k + 1), iln = tab_inv4(t, k + 1);
+        float4 bn = reversed(ld(nq - 2 - k));
+        const float4 grn = tab_g4(tr, k + 1), irn = tab_inv4(tr, k + 1);
+        if (k == 0) bn.x += fold1;
+        dl = fwd4(a, gl, il, dl);
+        dr = fwd4(b, gr, ir, dr);
+        st(k, a);
+        st(nq - 1 - k, reversed(b));
+        a = an;
+        b = bn;
+        gl = gln;
+        il = iln;
+        gr = grn;
+        ir = irn;
     }
-    for (; q - 1 >= 1; q -= 2) {   // a holds whole chunk q
-        float4 b = ld(q - 1), gb = tab_g4(t, q - 1);
-        x = bwd4(a, ga, x);
-        st(q, a);
-        a = ld(q - 2);
-        ga = tab_g4(t, q - 2);
-        x = bwd4(b, gb, x);
-        st(q - 1, b);
+    for (; k + 1 < hr; ++k) {   // gl, il: the constants from here on
+        const float4 an = ld(k + 1), bn = reversed(ld(nq - 2 - k));
+        dl = fwd4(a, gl, il, dl);
+        dr = fwd4(b, gl, il, dr);
+        st(k, a);
+        st(nq - 1 - k, reversed(b));
+        a = an;
+        b = bn;
     }
-    if (q >= 1) {   // q == 1
-        float4 b = ld(0), gb = tab_g4(t, 0);
-        x = bwd4(a, ga, x);
-        st(1, a);
-        x = bwd4p(b, gb, x, 1, 3);
-        st(0, b);
-    } else {        // a holds chunk 0
-        x = bwd4p(a, ga, x, 1, 3);
-        st(0, a);
+    // the innermost chunks stay in registers
+    dl = fwd4(a, gl, il, dl);
+    dr = fwd4(b, gr, ir, dr);
+    float4 g = gl;
+    if (hl > hr) {
+        const float4 an = ld(hr);
+        st(hr - 1, a);
+        a = an;
+        g = tab_g4(t, hr);
+        dl = fwd4(a, g, tab_inv4(t, hr), dl);
     }
+    float xl = fmaf(tj[1], dl, dr) * tj[2];   // the right half's first value, from both sides
+    float xr = fmaf(tj[0], dr, dl) * tj[2];   // the left half's last
+    if (hl > hr) {
+        const float4 an = ld(hr - 1);
+        xl = bwd4(a, g, xl);
+        st(hr, a);
+        a = an;
+    }
+    k = hr - 1;
+    for (; k > 0 && k >= kc; --k) {
+        const float4 an = ld(k - 1), bn = reversed(ld(nq - k));
+        xl = bwd4(a, gl, xl);
+        xr = bwd4(b, gl, xr);
+        st(k, a);
+        st(nq - 1 - k, reversed(b));
+        a = an;
+        b = bn;
+    }
+    gl = tab_g4(t, k);
+    gr = tab_g4(tr, k);
+    for (; k > 0; --k) {
+        const float4 an = ld(k - 1), bn = reversed(ld(nq - k)), gln = tab_g4(t, k - 1), grn = tab_g4(tr, k - 1);
+        xl = bwd4(a, gl, xl);
+        xr = bwd4(b, gr, xr);
+        st(k, a);
+        st(nq - 1 - k, reversed(b));
+        a = an;
+        b = bn;
+        gl = gln;
+        gr = grn;
+    }
+    bwd4(a, gl, xl);
+    bwd4(b, gr, xr);
+    a.x = lo;
+    b.x = b0.x;   // the places up to the end node as they were
+    b.y = lead >= 1 ? b0.y : b.y;
+    b.z = lead >= 2 ? b0.z : b.z;
+    b.w = lead == 3 ? b0.w : b.w;
+    st(0, a);
+    st(nq - 1, reversed(b));
 }
 
 // x tile through the row tensor map: lane t solves line t stored at
@@ -378,13 +422,10 @@ __device__ __forceinline__ void thomas_line(const float* t, int n, LD ld, ST st)
 __device__ __forceinline__ void row_line(float* row, const LineRule& r, const float* t)
 {
     const int n = static_cast<int>(r.n);
-    if (n >= 3) {
-        row[1] += r.fold;
-        if (n > 3) row[n - 2] += r.fold;
-        thomas_line(
-            t, n, [row](int q) { return *reinterpret_cast<const float4*>(row + 4 * q); },
+    if (n >= 3)
+        split_line(
+            t, n, r.fold, [row](int q) { return *reinterpret_cast<const float4*>(row + 4 * q); },
             [row](int q, float4 v) { *reinterpret_cast<float4*>(row + 4 * q) = v; });
-    }
     if (r.dir) {
         row[0] = r.T;
         row[n - 1] = r.T;
@@ -408,11 +449,9 @@ __device__ __forceinline__ void solve_cols(float* st, const SweepTile& tile, con
         for (int j = 0; j < n; ++j) c[j * 32] = r.T;   // applyDirichletBC fused: the line lies on a face
         return;
     }
-    if (n >= 3) {
-        c[32] += r.fold;
-        if (n > 3) c[(n - 2) * 32] += r.fold;
-        thomas_line(
-            t, n,
+    if (n >= 3)
+        split_line(
+            t, n, r.fold,
             [c](int q) {
                 return make_float4(c[(4 * q) * 32], c[(4 * q + 1) * 32], c[(4 * q + 2) * 32], c[(4 * q + 3) * 32]);
             },
@@ -422,7 +461,6 @@ __device__ __forceinline__ void solve_cols(float* st, const SweepTile& tile, con
                 c[(4 * q + 2) * 32] = v.z;
                 c[(4 * q + 3) * 32] = v.w;
             });
-    }
     if (r.dir) {
         c[0] = r.T;
         c[(n - 1) * 32] = r.T;
@@ -522,29 +560,24 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tma(const SweepTile* __restric
 // ------------------------------------------------------- fused x + y sweeps of a plane
 
 // Column line of a plane in shared memory (rows P floats apart): the steps
-// of solve_cols with row stride P.  'face': the line lies on an x face of a
-// 2-D block whose last sweep this is, so applyDirichletBC sets it to T.
-__device__ __forceinline__ void plane_col(float* c, int P, const LineRule& r, const float* t, bool face)
+// of solve_cols with row stride P.
+__device__ __forceinline__ void plane_col(float* c, int P, const LineRule& r, const float* t)
 {
     const int n = static_cast<int>(r.n);
-    if (face) {
-        for (int j = 0; j < n; ++j) c[j * P] = r.T;
-        return;
-    }
-    if (n >= 3) {
-        c[P] += r.fold;
-        if (n > 3) c[(n - 2) * P] += r.fold;
-        auto ld = [c, P](int q) {
-            return make_float4(c[(4 * q) * P], c[(4 * q + 1) * P], c[(4 * q + 2) * P], c[(4 * q + 3) * P]);
-        };
-        auto st4 = [c, P](int q, float4 v) {
-            c[(4 * q) * P] = v.x;
-            c[(4 * q + 1) * P] = v.y;
-            c[(4 * q + 2) * P] = v.z;
-            c[(4 * q + 3) * P] = v.w;
-        };
-        thomas_line(t, n, ld, st4);
-    }
+    if (n >= 3)
+        split_line(
+            t, n, r.fold,
+            [c, P](int q) {
+                const float* p = c + 4 * q * P;
+                return make_float4(p[0], p[P], p[2 * P], p[3 * P]);
+            },
+            [c, P](int q, float4 v) {
+                float* p = c + 4 * q * P;
+                p[0] = v.x;
+                p[P] = v.y;
+                p[2 * P] = v.z;
+                p[3 * P] = v.w;
+            });
     if (r.dir) {
         c[0] = r.T;
         c[(n - 1) * P] = r.T;
@@ -555,17 +588,27 @@ __device__ __forceinline__ void plane_col(float* c, int P, const LineRule& r, co
 // (rows of pitch P = row_smem_pitch(nx), zero-filled past nx) and both
 // rules' tables come in with one tensor box and two bulk copies; every row
 // is solved (x sweep), then every column (y sweep), and the plane goes back
-// with one tensor store.  The steps on each line are those of the x and y
-// tile kernels, so the result is the same bits, but the plane crosses HBM
-// once for both sweeps.  Several CTAs per SM overlap one plane's copies
-// with another's solves, and each CTA prefetches into L2 (a tensor-box
-// prefetch, no shared memory) the plane of the CTA 'ahead' jobs later, so
-// that CTA's load is served from L2.
-__global__ void __launch_bounds__(kPlaneThreads) k_sweep_planes(const PlaneJob* __restrict__ jobs,
-                                                                const float* __restrict__ tab,
-                                                                const void* __restrict__ tmaps, int apply_faces,
-                                                                const uint8_t* __restrict__ mask,
-                                                                unsigned* __restrict__ status, uint32_t ahead)
+// with one tensor store.  ZK: x-z planes, columns only.  The steps on each
+// line are those of the x and y tile kernels, so the result is the same
+// bits, but the plane crosses HBM once for both sweeps.  Several CTAs per
+// SM overlap one plane's copies with another's solves, and each CTA
+// prefetches into L2 (a tensor-box prefetch, no shared memory) the plane of
+// the CTA 'ahead' jobs later, so that CTA's load is served from L2.
+//
+// What bounds it: the x + y pass by the shared-memory wavefronts of its two
+// solves beside HBM, the z pass by HBM.  Per chunk of a warp's lines a solve
+// moves 16 wavefronts of values and, until g settles, 3 of table; keeping
+// the settled g and 1 / den in registers took the 120^3 x + y pass from
+// 75.1 to 65.9 us (332 MB, 5.0 TB/s; z 54.8 us, 6.1 TB/s), with 80 registers
+// 80^3 from 68.4 to 60.6 and 48^3 from 56.8 to 50.5; four 150^3 fields 73.3 +
+// 55.5 -> 57.6 + 45.9 us (one thread per line, not 128).  Measured and not
+// taken: a line's chunks held in registers between the passes (fewer
+// wavefronts, but unrolled code starves on instruction fetch: 120^3 79 us),
+// half a line per thread with the halves in two warps (66-89 us).
+template <bool ZK>
+__global__ void __launch_bounds__(256, 3)
+    k_sweep_planes(const PlaneJob* __restrict__ jobs, const float* __restrict__ tab, const void* __restrict__ tmaps,
+                   int apply_faces, const uint8_t* __restrict__ mask, unsigned* __restrict__ status, uint32_t ahead)
 {
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem);
@@ -573,10 +616,9 @@ __global__ void __launch_bounds__(kPlaneThreads) k_sweep_planes(const PlaneJob* 
     const PlaneJob jb = jobs[blockIdx.x];
     const uint32_t ii = jb.inst & kPlaneInstMask;
     if (mask && !(mask[ii] & STEP_DIFFUSE)) return;   // the whole CTA leaves together
-    const bool zk = (jb.inst & kPlaneZ) != 0;
-    const uint32_t nx = jb.nx, ny = jb.ny, P = plane_pitch(nx, zk);
-    float* tx = pl + plane_data_floats(nx, ny, zk);
-    float* ty = zk ? tx : tx + tab_floats(nx);
+    const uint32_t nx = jb.nx, ny = jb.ny, P = plane_pitch(nx, ZK);
+    float* tx = pl + plane_data_floats(nx, ny, ZK);
+    float* ty = ZK ? tx : tx + tab_floats(nx);
     const void* map = static_cast<const unsigned char*>(tmaps) + static_cast<size_t>(jb.map) * 128;
     if (threadIdx.x == 0) {
         mbar_init(bar, 1);
@@ -584,9 +626,9 @@ __global__ void __launch_bounds__(kPlaneThreads) k_sweep_planes(const PlaneJob* 
     }
     __syncthreads();
     if (threadIdx.x == 0) {
-        const uint32_t tbx = zk ? 0u : tab_floats(nx) * 4u, tby = tab_floats(ny) * 4u;
+        const uint32_t tbx = ZK ? 0u : tab_floats(nx) * 4u, tby = tab_floats(ny) * 4u;
         mbar_arrive_expect_tx(bar, P * ny * 4u + tbx + tby);   // the whole box, fill included
-        if (zk) {
+        if (ZK) {
             tensor_load3(pl, map, 0, static_cast<int>(jb.row0), 0, bar);
         } else {
             tensor_load2(pl, map, 0, static_cast<int>(jb.row0), bar);
@@ -600,7 +642,7 @@ __global__ void __launch_bounds__(kPlaneThreads) k_sweep_planes(const PlaneJob* 
             const PlaneJob nj = jobs[blockIdx.x + ahead];
             if (!mask || (mask[nj.inst & kPlaneInstMask] & STEP_DIFFUSE)) {
                 const void* nmap = static_cast<const unsigned char*>(tmaps) + static_cast<size_t>(nj.map) * 128;
-                if (nj.inst & kPlaneZ) tensor_prefetch3(nmap, 0, static_cast<int>(nj.row0), 0);
+                if (ZK) tensor_prefetch3(nmap, 0, static_cast<int>(nj.row0), 0);
                 else tensor_prefetch2(nmap, 0, static_cast<int>(nj.row0));
             }
         }
@@ -627,20 +669,26 @@ __global__ void __launch_bounds__(kPlaneThreads) k_sweep_planes(const PlaneJob* 
     ry.fold = jb.fold_y;
     ry.T = jb.T_y;
     ry.dir = (jb.inst & kPlaneDirY) ? 1u : 0u;
-    if (!zk) {
+    if (!ZK) {
         for (uint32_t r = threadIdx.x; r < ny; r += blockDim.x) row_line(pl + r * P, rx, tx);
         __syncthreads();
     }
-    // faces of the block's last sweep (2-D: y, 3-D: z): x faces, and a whole
-    // z plane on a y face
+    // faces of the block's last sweep (2-D: y, 3-D: z; applyDirichletBC): x
+    // faces, and a whole z plane on a y face
     const bool faces = apply_faces && (jb.inst & kPlaneFaces) != 0;
-    const bool slab_face = (jb.inst & kPlaneSlabFace) != 0;
-    for (uint32_t c = threadIdx.x; c < nx; c += blockDim.x)
-        plane_col(pl + c, static_cast<int>(P), ry, ty, faces && (slab_face || c == 0u || c + 1u == nx));
+    const bool slab_face = faces && (jb.inst & kPlaneSlabFace) != 0;
+    if (!slab_face)
+        for (uint32_t c = threadIdx.x; c < nx; c += blockDim.x) plane_col(pl + c, static_cast<int>(P), ry, ty);
+    if (faces) {
+        __syncthreads();
+        const uint32_t step = slab_face ? 1u : (nx > 1 ? nx - 1 : 1u);   // every column, or the first and the last
+        for (uint32_t j = threadIdx.x; j < ny; j += blockDim.x)
+            for (uint32_t c = 0; c < nx; c += step) pl[j * P + c] = ry.T;
+    }
     fence_async_smem();
     __syncthreads();
     if (threadIdx.x == 0) {
-        if (zk) tensor_store3(map, 0, static_cast<int>(jb.row0), 0, pl);
+        if (ZK) tensor_store3(map, 0, static_cast<int>(jb.row0), 0, pl);
         else tensor_store2(map, 0, static_cast<int>(jb.row0), pl);
         bulk_commit();
         bulk_wait_read<0>();   // shared memory may be released once the store has read it
@@ -724,7 +772,7 @@ __global__ void __launch_bounds__(32 * kLongLines) k_sweep_long(float* __restric
     if (!tile_on(r, mask)) return;   // the whole CTA leaves together
     const int n = static_cast<int>(r.n), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool rows = (tile.face & TILE_ROWS) != 0;
-    const float* t = tab + r.tab;
+    const float* t = tab + r.tab + seq_table_offset(r.n);
     // the line and position a thread moves at step i: rows, one line per
     // warp; columns, 8 adjacent lines per row of threads
     const int line = rows ? warp : static_cast<int>(threadIdx.x & 7u);
@@ -1015,42 +1063,41 @@ bool encode_xz_plane_map(void* map128, float* block, uint32_t nx, uint32_t ny, u
 
 size_t sweep_planes_smem(uint32_t floats) { return 128 + static_cast<size_t>(floats) * sizeof(float); }
 
-cudaError_t sweep_planes_prepare()
+static const void* plane_kernel(bool z)
 {
-    const void* fn = reinterpret_cast<const void*>(k_sweep_planes);
-    cudaError_t e = allow_max_smem(fn);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    return e;
+    return z ? reinterpret_cast<const void*>(&k_sweep_planes<true>) : reinterpret_cast<const void*>(&k_sweep_planes<false>);
 }
 
-int sweep_planes_ctas(uint32_t floats)
+cudaError_t sweep_planes_prepare()
+{
+    for (bool z : {false, true}) {
+        cudaError_t e = allow_max_smem(plane_kernel(z));
+        if (e == cudaSuccess)
+            e = cudaFuncSetAttribute(plane_kernel(z), cudaFuncAttributePreferredSharedMemoryCarveout,
+                                     cudaSharedmemCarveoutMaxShared);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
+}
+
+int sweep_planes_ctas(bool z, int threads, uint32_t floats)
 {
     int n = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_sweep_planes, kPlaneThreads, sweep_planes_smem(floats)) !=
-        cudaSuccess)
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, plane_kernel(z), threads, sweep_planes_smem(floats)) !=
+        cudaSuccess) {
+        cudaGetLastError();
         return 0;
+    }
     return n;
 }
 
-cudaError_t launch_sweep_planes(cudaStream_t st, const PlaneJob* jobs, uint32_t njobs, const float* tab,
-                                const void* tmaps, uint32_t floats, int apply_faces, const uint8_t* mask,
-                                unsigned* status)
+cudaError_t launch_sweep_planes(cudaStream_t st, bool z, int threads, const PlaneJob* jobs, uint32_t njobs,
+                                const float* tab, const void* tmaps, uint32_t floats, int apply_faces,
+                                const uint8_t* mask, unsigned* status, uint32_t ahead)
 {
     if (njobs == 0) return cudaSuccess;
-    // prefetch distance: a quarter of the CTAs of this launch resident at
-    // once (measured: a half, one or two residencies ahead gain less or lose).
-    // The SM count is read once, on the first device used; it only sets this
-    // distance, never which data is read.
-    static const int sms = [] {
-        int dev = 0, n = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
-            n = 1;
-        return n;
-    }();
-    const uint32_t ahead = static_cast<uint32_t>(sweep_planes_ctas(floats) * sms / 4);
-    k_sweep_planes<<<njobs, kPlaneThreads, sweep_planes_smem(floats), st>>>(jobs, tab, tmaps, apply_faces, mask,
-                                                                            status, ahead);
+    if (z) k_sweep_planes<true><<<njobs, threads, sweep_planes_smem(floats), st>>>(jobs, tab, tmaps, apply_faces, mask, status, ahead);
+    else k_sweep_planes<false><<<njobs, threads, sweep_planes_smem(floats), st>>>(jobs, tab, tmaps, apply_faces, mask, status, ahead);
     return cudaGetLastError();
 }
 

@@ -31,8 +31,6 @@ enum Field : int {
 //   backward  rho_i = d_i - c'_i rho_{i+1}
 // with den_i = b + c c'_{i-1}, c'_i = -c / den_i = -g_i; written as
 // d_i = fma(g_i, d_{i-1}, (rho_i + fold_i) * inv_i), x_i = fma(g_i, x_{i+1}, d_i).
-// Table layout: line positions in chunks of 4, chunk q at tab + 8 q holds
-// {g[4q..4q+3], inv[4q..4q+3]} (32-byte aligned; zero at the end nodes).
 struct LineRule {
     uint32_t tab;   // first float of the rule's table (multiple of 8)
     uint32_t n;     // line length
@@ -44,8 +42,34 @@ struct LineRule {
     uint32_t _pad;
 };
 
-// Floats of table for a line of n positions.
-__host__ __device__ constexpr uint32_t tab_floats(uint32_t n) { return ((n + 3u) / 4u) * 8u; }
+// Longest line the split tables serve (tensor-map boxes are at most 256).
+constexpr uint32_t kTensorMaxN = 256;
+
+// Table of a line solved from both ends (n <= kTensorMaxN): the line's nq
+// chunks of 4 positions are split into hl left ones and nq - hl right ones.
+// Floats [0, 8 hl): the left half, chunk k {g[4k..4k+3], inv[4k..4k+3]};
+// [8 hl, 16 hl): the right half, position p at index 4 nq - 1 - p (the end
+// node at 4 nq - n); then, in the middle's 8 floats, g of the left half's
+// last and of the right half's innermost position (0 where the right half
+// has no interior node), 1 / (1 - their product), and (bits) the first chunk
+// from which every entry of both halves is the same.  Zero at the end nodes
+// and past the line.  The left half's last value x_m and the right half's
+// first x_{m+1} follow from x_m = d_m + g_m x_{m+1}, x_{m+1} = d'_{m+1} +
+// g'_{m+1} x_m.
+struct SplitTable {
+    int n, nq, hl;
+    __host__ __device__ constexpr explicit SplitTable(int n_) : n(n_), nq((n_ + 3) / 4), hl(((n_ + 3) / 4 + 1) / 2) {}
+    __host__ __device__ constexpr int right() const { return 8 * hl; }
+    __host__ __device__ constexpr int middle() const { return 16 * hl; }
+    __host__ __device__ constexpr int floats() const { return 16 * hl + 8; }
+    __host__ __device__ constexpr bool right_has_interior() const { return n - 2 >= 4 * hl; }
+};
+// Floats of the table a tile or plane stages for a line of n positions.
+__host__ __device__ constexpr uint32_t tab_floats(uint32_t n) { return static_cast<uint32_t>(SplitTable(static_cast<int>(n)).floats()); }
+// The sequential table (one-warp-per-line kernel: position i at chunk i / 4,
+// {g[4], inv[4]}) follows the split one where a line has both.
+__host__ __device__ constexpr uint32_t seq_table_offset(uint32_t n) { return n <= kTensorMaxN ? tab_floats(n) : 0u; }
+__host__ __device__ constexpr uint32_t seq_table_floats(uint32_t n) { return ((n + 3u) / 4u) * 8u; }
 
 // A tile of lines for one sweep launch.  Row tiles (x sweep, TILE_ROWS):
 // 'count' (<= 32) lines of length n starting at element 'base', lines 'rs'
@@ -80,8 +104,6 @@ struct SweepTile {
 static_assert(sizeof(SweepTile) == 64, "one 64-byte descriptor per tile");
 enum : uint32_t { TILE_FACE = 1u, TILE_ROWS = 4u, TILE_TENSOR = 8u, TILE_AXIS_Z = 16u };
 
-// Longest line a tensor-map box can cover (box dimensions are <= 256).
-constexpr uint32_t kTensorMaxN = 256;
 // Tensor-map slots per rule: x rules use slot 0, y / z rules one per
 // column-tile width (32, 16, 8).
 constexpr uint32_t kMapsPerRule = 4;
@@ -156,7 +178,9 @@ constexpr uint32_t kPlaneDirX = 1u << 31, kPlaneDirY = 1u << 30, kPlaneFaces = 1
 constexpr uint32_t kPlaneZ = 1u << 28;          // an x-z plane of z lines
 constexpr uint32_t kPlaneSlabFace = 1u << 27;   // z job: the plane is a y face of the block
 constexpr uint32_t kPlaneInstMask = (1u << 27) - 1u;
-constexpr uint32_t kPlaneThreads = 128;
+// Threads of a plane CTA: one per line of the longer side, at most 256.  (A
+// fixed 128 left 22 lines of a 150-voxel plane to a second round.)
+constexpr int plane_threads(uint32_t side) { return side >= 256u ? 256 : static_cast<int>((side + 31u) / 32u) * 32; }
 // Row pitch of a plane in shared memory: x-y planes row_smem_pitch(nx) (the
 // rows are solved with 16-byte accesses), z planes nx rounded up to 4.
 __host__ __device__ constexpr uint32_t plane_pitch(uint32_t nx, bool z)
@@ -183,19 +207,20 @@ size_t sweep_tma_smem(int warps, int nstages, int stage_floats);
 int sweep_tma_occupancy(bool rows, int warps, int nstages, int stage_floats);   // CTAs per SM (0 = does not fit)
 // tmaps: the 128-byte CUtensorMaps the tiles name (64-byte aligned, global
 // memory); every tile is flagged TILE_TENSOR.
-// Fused x + y sweeps, one CTA per plane; 'floats' = the largest
-// plane_floats of the jobs.
-cudaError_t launch_sweep_planes(cudaStream_t st, const PlaneJob* jobs, uint32_t njobs, const float* tab,
-                                const void* tmaps, uint32_t floats, int apply_faces, const uint8_t* mask,
-                                unsigned* status);
-// Lets the plane kernel use the opt-in shared memory, with the largest
+// Fused x + y sweeps (z: x-z planes of z lines), one CTA of 'threads' per
+// plane; 'floats' = the largest plane_floats of the jobs, 'ahead' = the L2
+// prefetch distance in jobs.
+cudaError_t launch_sweep_planes(cudaStream_t st, bool z, int threads, const PlaneJob* jobs, uint32_t njobs,
+                                const float* tab, const void* tmaps, uint32_t floats, int apply_faces,
+                                const uint8_t* mask, unsigned* status, uint32_t ahead);
+// Lets the plane kernels use the opt-in shared memory, with the largest
 // shared-memory carveout, so launches of every plane size share one SM
-// configuration (current device; once per device, outside stream capture).
+// configuration (current device, outside stream capture).
 cudaError_t sweep_planes_prepare();
 size_t sweep_planes_smem(uint32_t floats);
 // Plane CTAs an SM holds at once for planes of 'floats' (0 = does not fit);
 // sweep_planes_prepare() first.
-int sweep_planes_ctas(uint32_t floats);
+int sweep_planes_ctas(bool z, int threads, uint32_t floats);
 bool encode_plane_map(void* map128, float* block, uint32_t nx, uint32_t ny, uint64_t rows, uint32_t px);
 bool encode_xz_plane_map(void* map128, float* block, uint32_t nx, uint32_t ny, uint32_t nz, uint32_t px);
 cudaError_t launch_sweep_tma(cudaStream_t st, bool rows, const SweepTile* tiles, uint32_t ntiles,

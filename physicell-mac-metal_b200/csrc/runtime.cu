@@ -323,10 +323,9 @@ void Tuner::save(const std::string& path)
 
 // ------------------------------------------------------------------ diffusion
 
-// Largest plane (with its tables) the fused x + y kernel takes: two CTAs
-// per SM fit the 227 KB of shared memory.
-static constexpr size_t kPlaneMaxSmem = 112 * 1024;
-
+// Largest plane (with its tables) the plane kernel takes: what a CTA may
+// hold of an SM's shared memory.
+static constexpr size_t kPlaneMaxSmem = 227 * 1024;
 
 static uint32_t axis_n(const pcg_grid_params& g, int a) { return a == 0 ? g.nx : (a == 1 ? g.ny : g.nz); }
 static float axis_h(const pcg_grid_params& g, int a) { return a == 0 ? g.dx : (a == 1 ? g.dy : g.dz); }
@@ -386,32 +385,68 @@ int Diffusion::build(pcg_ctx* c, std::vector<DiffInstance> instances)
                 r.T = sp.target_value;
                 r.dir = dir ? 1u : 0u;
                 r.inst = static_cast<uint32_t>(i);
-                h_tab_.resize(h_tab_.size() + tab_floats(std::max<uint32_t>(n, 1)), 0.f);
-                float* tb = h_tab_.data() + r.tab;
-                // position i: g_i = c / den_i = -c'_i and 1 / den_i (chunked layout)
-                auto put = [tb](uint32_t i, double g, double inv) {
-                    tb[(i / 4) * 8 + i % 4] = static_cast<float>(g);
-                    tb[(i / 4) * 8 + 4 + i % 4] = static_cast<float>(inv);
-                };
+                h_tab_.resize(h_tab_.size() + seq_table_offset(n) + seq_table_floats(n), 0.f);
+                // g_i = c / den_i = -c'_i and 1 / den_i of every position, in FP64
+                std::vector<double> gs(n, 0.0), is(n, 0.0);
                 // the end interior nodes' diagonal: the reference's 1 + c + hd
                 // (diffusion_2d.metal:48), or with the consistent Dirichlet
                 // option the interior one on Dirichlet lines
                 const double b_int = 1.0 + 2.0 * cc + hd;
                 const double b_bnd = (dir && sp.dirichlet_consistent) ? b_int : 1.0 + cc + hd;
                 if (n == 3) {
-                    put(1, 0.0, 1.0 / b_int);
+                    is[1] = 1.0 / b_int;
                     r.fold = dir ? static_cast<float>(2.0 * cc * T) : 0.f;
                 } else if (n >= 4) {
-                    double cp = -cc / b_bnd;
-                    put(1, -cp, 1.0 / b_bnd);
-                    for (uint32_t m = 2; m + 2 < n; ++m) {
-                        const double den = b_int + cc * cp;
+                    double cp = 0.0;
+                    for (uint32_t m = 1; m + 1 < n; ++m) {
+                        const double den = (m == 1 || m + 2 == n ? b_bnd : b_int) + cc * cp;
                         cp = -cc / den;
-                        put(m, -cp, 1.0 / den);
+                        gs[m] = -cp;
+                        is[m] = 1.0 / den;
                     }
-                    const double den = b_bnd + cc * cp;
-                    put(n - 2, cc / den, 1.0 / den);
                     r.fold = dir ? static_cast<float>(cc * T) : 0.f;
+                }
+                // entry i of a chunked table
+                auto put = [](float* tb, uint32_t i, double g, double inv) {
+                    tb[(i / 4) * 8 + i % 4] = static_cast<float>(g);
+                    tb[(i / 4) * 8 + 4 + i % 4] = static_cast<float>(inv);
+                };
+                float* seq = h_tab_.data() + r.tab + seq_table_offset(n);
+                for (uint32_t m = 1; m + 1 < n; ++m) put(seq, m, gs[m], is[m]);
+                if (n <= kTensorMaxN) {
+                    // from both ends: the right half's coefficients are the
+                    // left ones counted from the right end
+                    const SplitTable st(static_cast<int>(n));
+                    float* tb = h_tab_.data() + r.tab;
+                    const uint32_t nl = 4u * static_cast<uint32_t>(st.hl);
+                    for (uint32_t m = 1; m + 1 < n && m < nl; ++m) put(tb, m, gs[m], is[m]);
+                    float* mid = tb + st.middle();
+                    mid[2] = 1.f;
+                    if (st.right_has_interior()) {
+                        const uint32_t lead = 4u * static_cast<uint32_t>(st.nq) - n;
+                        for (uint32_t e = 1; n - 1 - e >= nl; ++e) put(tb + st.right(), lead + e, gs[e], is[e]);
+                        const double gl = gs[nl - 1], gr = gs[n - 1 - nl];
+                        mid[0] = static_cast<float>(gl);
+                        mid[1] = static_cast<float>(gr);
+                        mid[2] = static_cast<float>(1.0 / (1.0 - gl * gr));
+                    }
+                    // g_i settles to the matrix's fixed point within a few
+                    // chunks: from the first chunk where every entry of both
+                    // halves is the same pair of floats, the solve keeps it
+                    // in registers
+                    const int hr = st.nq - st.hl;
+                    auto settled = [&](int k) {
+                        const float* c = tb + 8 * (st.hl - 1);
+                        for (int u = 0; u < 4; ++u)
+                            for (int half = 0; half < (k < hr ? 2 : 1); ++half) {
+                                const float* e = tb + half * st.right() + 8 * k;
+                                if (e[u] != c[0] || e[4 + u] != c[4]) return false;
+                            }
+                        return true;
+                    };
+                    int kc = st.hl;
+                    while (kc > 1 && settled(kc - 1)) --kc;
+                    std::memcpy(mid + 3, &kc, sizeof kc);
                 }
                 rule_index_.push_back(static_cast<uint32_t>(h_rules_.size()));
                 h_rules_.push_back(r);
@@ -512,13 +547,11 @@ int Diffusion::build(pcg_ctx* c, std::vector<DiffInstance> instances)
     return build_planes();
 }
 
-// Plane jobs grouped by shared-memory size, so small planes are not charged
-// the largest plane's footprint; largest planes first.
 // Plane lists from per-class jobs: runs of 'merge' consecutive non-empty
 // classes (0: all of them) become one list, launched with the largest
 // plane's shared memory.
-static int plane_lists(pcg_ctx* ctx, const std::vector<PlaneJob>* jobs, const uint32_t* fl, const uint64_t* un,
-                       int classes, int merge, std::vector<PlaneList>& out)
+static int plane_lists(pcg_ctx* ctx, bool z, const std::vector<PlaneJob>* jobs, const uint32_t* fl, const int* thr,
+                       const uint64_t* un, int classes, int merge, std::vector<PlaneList>& out)
 {
     std::vector<int> used;
     for (int c = classes - 1; c >= 0; --c)
@@ -533,9 +566,14 @@ static int plane_lists(pcg_ctx* ctx, const std::vector<PlaneJob>* jobs, const ui
             const int c = used[k];
             all.insert(all.end(), jobs[c].begin(), jobs[c].end());
             pl.floats = std::max(pl.floats, fl[c]);
+            pl.threads = std::max(pl.threads, thr[c]);
             pl.units += un[c];
         }
         pl.n = static_cast<uint32_t>(all.size());
+        pl.z = z;
+        // prefetch distance: a quarter of the CTAs of this launch resident at
+        // once (measured: a half, one or two residencies ahead gain less or lose)
+        pl.ahead = static_cast<uint32_t>(sweep_planes_ctas(z, pl.threads, pl.floats) * ctx->sms / 4);
         PCG_CU(ctx, pl.jobs.alloc(all.size() * sizeof(PlaneJob)));
         PCG_CU(ctx, cudaMemcpyAsync(pl.jobs.p, all.data(), all.size() * sizeof(PlaneJob), cudaMemcpyHostToDevice,
                                     ctx->stream));
@@ -547,8 +585,10 @@ static int plane_lists(pcg_ctx* ctx, const std::vector<PlaneJob>* jobs, const ui
 int Diffusion::regroup_planes(int merge)
 {
     plane_merge = merge;
-    PCG_TRY(plane_lists(ctx, cls_jobs_[0], cls_floats_[0], cls_units_[0], kPlaneClasses, merge, planes));
-    PCG_TRY(plane_lists(ctx, cls_jobs_[1], cls_floats_[1], cls_units_[1], kPlaneClasses, merge, zplanes));
+    PCG_TRY(plane_lists(ctx, false, cls_jobs_[0], cls_floats_[0], cls_threads_[0], cls_units_[0], kPlaneClasses, merge,
+                        planes));
+    PCG_TRY(plane_lists(ctx, true, cls_jobs_[1], cls_floats_[1], cls_threads_[1], cls_units_[1], kPlaneClasses, merge,
+                        zplanes));
     return PCG_OK;
 }
 
@@ -563,12 +603,18 @@ int Diffusion::build_planes()
     bool any = false;
     for (size_t i = 0; i < inst.size(); ++i) any = any || plane_inst_[i] || zplane_inst_[i];
     if (any) PCG_CU(ctx, sweep_planes_prepare());   // before the occupancy queries
-    // Classes by the plane CTAs an SM holds for the plane's shared memory
-    // (class kMaxCtas - k for k CTAs), so each plane runs at the occupancy
-    // its own size allows; a class launches with its largest plane's size,
-    // which by construction allows the same k.
+    // Classes by the plane CTAs an SM holds for the plane's size (class
+    // kMaxCtas - k for k CTAs), so each plane runs at the occupancy its own
+    // size allows; a class launches with its largest plane's size, which by
+    // construction allows the same k.
     constexpr int kMaxCtas = kPlaneClasses;
-    auto cls = [&](uint32_t pf) { return kMaxCtas - std::min(std::max(sweep_planes_ctas(pf), 1), kMaxCtas); };
+    std::map<std::pair<int, uint32_t>, int> known[2];   // (threads, floats) -> class: one query per plane size
+    auto cls = [&](bool z, int threads, uint32_t pf) {
+        const auto key = std::make_pair(threads, pf);
+        const auto it = known[z].find(key);
+        if (it != known[z].end()) return it->second;
+        return known[z][key] = kMaxCtas - std::min(std::max(sweep_planes_ctas(z, threads, pf), 1), kMaxCtas);
+    };
     std::vector<PlaneJob>* jobs = cls_jobs_[0];
     std::vector<PlaneJob>* zjobs = cls_jobs_[1];
     uint32_t* fl = cls_floats_[0];
@@ -579,6 +625,7 @@ int Diffusion::build_planes()
         jobs[c].clear();
         zjobs[c].clear();
         fl[c] = zfl[c] = 0;
+        cls_threads_[0][c] = cls_threads_[1][c] = 0;
         un[c] = zun[c] = 0;
     }
     for (size_t i = 0; i < inst.size(); ++i) {
@@ -586,7 +633,9 @@ int Diffusion::build_planes()
         const uint32_t nx = d.g.nx, ny = d.g.ny, nz = d.g.nz;
         if (plane_inst_[i]) {
             const uint32_t pf = plane_floats(nx, ny);
-            const int c = cls(pf);
+            const int thr = plane_threads(std::max(nx, ny));
+            const int c = cls(false, thr, pf);
+            cls_threads_[0][c] = std::max(cls_threads_[0][c], thr);
             for (uint32_t s = 0; s < d.g.n_substrates; ++s) {
                 const uint32_t rx_i = rule_of(i, s, 0);
                 const LineRule& rx = h_rules_[rx_i];
@@ -613,7 +662,9 @@ int Diffusion::build_planes()
         }
         if (zplane_inst_[i]) {
             const uint32_t pf = plane_floats(nx, nz, true);
-            const int c = cls(pf);
+            const int thr = plane_threads(nx);
+            const int c = cls(true, thr, pf);
+            cls_threads_[1][c] = std::max(cls_threads_[1][c], thr);
             for (uint32_t s = 0; s < d.g.n_substrates; ++s) {
                 const uint32_t rz_i = rule_of(i, s, 2);
                 const LineRule& rz = h_rules_[rz_i];
@@ -879,8 +930,8 @@ int Diffusion::launch_planes(const std::vector<PlaneList>& pls, bool fuse, const
     for (size_t k = 0; k < pls.size(); ++k) {
         const PlaneList& pl = pls[k];
         const cudaStream_t st = k == 0 ? ctx->stream : ctx->fork_st[(k - 1) % side];
-        cudaError_t e = launch_sweep_planes(st, pl.jobs.as<PlaneJob>(), pl.n, tab.as<float>(), tmaps.p, pl.floats,
-                                            fuse ? 1 : 0, mask, ctx->status);
+        cudaError_t e = launch_sweep_planes(st, pl.z, pl.threads, pl.jobs.as<PlaneJob>(), pl.n, tab.as<float>(), tmaps.p,
+                                            pl.floats, fuse ? 1 : 0, mask, ctx->status, pl.ahead);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "plane sweep launch");
         ctx->launches++;
     }

@@ -161,11 +161,14 @@ struct DiffInstance {
     int ndim() const { return g.nz > 1 ? 3 : 2; }
 };
 
-// Plane jobs launched together: the planes whose shared memory allows the
-// same number of CTAs per SM, launched with the largest one's size.
+// Plane jobs launched together: the planes whose size allows the same number
+// of CTAs per SM, launched with the largest one's size.
 struct PlaneList {
     DevBuf jobs;
     uint32_t n = 0;
+    int threads = 0;           // per CTA (plane_threads of the largest side)
+    bool z = false;            // x-z planes
+    uint32_t ahead = 0;        // L2 prefetch distance (jobs)
     uint32_t floats = 0;       // largest plane_floats of the jobs
     uint64_t units = 0;        // voxel-substrates covered
 };
@@ -230,10 +233,12 @@ private:
     int build_axis(int axis, const std::vector<uint8_t>* skip, std::vector<SweepList>& ls);
     int build_planes();
     // plane jobs per occupancy class (class kPlaneClasses - k: k CTAs per
-    // SM), their largest plane and the voxel-substrates they cover
+    // SM), their largest plane, their threads and the voxel-substrates they
+    // cover
     static constexpr int kPlaneClasses = 32;
     std::vector<PlaneJob> cls_jobs_[2][kPlaneClasses];
     uint32_t cls_floats_[2][kPlaneClasses] = {};
+    int cls_threads_[2][kPlaneClasses] = {};
     uint64_t cls_units_[2][kPlaneClasses] = {};
     std::vector<uint8_t> plane_inst_;    // instance's x + y sweeps run as planes
     std::vector<uint8_t> zplane_inst_;   // instance's z sweep runs as x-z planes
