@@ -43,6 +43,8 @@ __global__ void k_sec_cell_consts(const float* __restrict__ soa, uint32_t stride
                                   const double* __restrict__ rates4, uint32_t n_rate, double dt,
                                   double* __restrict__ cc, uint32_t* __restrict__ flags)
 {
+    dependents_may_launch();
+    if (!await_predecessors()) return;
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     const bool live = g < n;
     const unsigned live_lanes = __ballot_sync(0xFFFFFFFFu, live);   // blocks are whole warps
@@ -85,6 +87,8 @@ __global__ void k_sec_permute(const uint32_t* __restrict__ skeys, const uint32_t
                               uint32_t invalid_key, const uint32_t* __restrict__ flags,
                               const double* __restrict__ cc, uint32_t n_rate, double* __restrict__ cs)
 {
+    dependents_may_launch();
+    if (!await_predecessors()) return;
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= n) return;
     if (skeys[q] >= invalid_key) return;
@@ -130,6 +134,8 @@ __global__ void __launch_bounds__(256, 6) k_secrete(float* __restrict__ dens, co
                           const CellInst* __restrict__ insts, const double* __restrict__ cs, uint64_t cap,
                           const uint32_t* __restrict__ flags, const uint8_t* __restrict__ mask)
 {
+    dependents_may_launch();
+    if (!await_predecessors()) return;
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= *n_runs) return;
     // a run's start and word (instance, the voxel's density element) were
@@ -230,6 +236,8 @@ __global__ void k_mech_bin(float* __restrict__ soa, uint32_t stride, uint32_t n,
                            uint32_t* __restrict__ slots, uint32_t* __restrict__ counts,
                            const uint8_t* __restrict__ mask)
 {
+    dependents_may_launch();
+    if (!await_predecessors()) return;
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n) return;
     const uint32_t ii = cell_inst[g];
@@ -262,6 +270,8 @@ __global__ void k_mech_place(const float* __restrict__ soa, uint32_t stride, con
                              const uint32_t* __restrict__ slots, const uint32_t* __restrict__ start, uint32_t n,
                              uint2* __restrict__ placed)
 {
+    dependents_may_launch();
+    if (!await_predecessors()) return;
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n) return;
     const float x = soa[static_cast<size_t>(F_POS_X) * stride + g];
@@ -313,6 +323,8 @@ __global__ void k_mech_order(const float* __restrict__ soa, uint32_t stride, con
                              const uint32_t* __restrict__ cell_inst, uint32_t* __restrict__ reach,
                              uint32_t* __restrict__ sorder, float4* __restrict__ spos, float4* __restrict__ sprm)
 {
+    dependents_may_launch();
+    if (!await_predecessors()) return;
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     const bool live = g < n;
     uint32_t ii = 0, rb = 0;
@@ -348,6 +360,8 @@ __global__ void k_mech_order(const float* __restrict__ soa, uint32_t stride, con
 __global__ void k_mech_stable_order(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ start,
                                     const uint2* __restrict__ placed, uint32_t n, uint32_t* __restrict__ sorder)
 {
+    dependents_may_launch();
+    if (!await_predecessors()) return;
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n) return;
     const uint32_t key = keys[g];
@@ -454,6 +468,8 @@ __global__ void __launch_bounds__(256, 5) k_mech_forces(const float4* __restrict
                                                      uint32_t* __restrict__ diag_hash,
                                                      const uint8_t* __restrict__ mask)
 {
+    dependents_may_launch();
+    if (!await_predecessors()) return;
     extern __shared__ uint32_t queue[];
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
@@ -603,6 +619,8 @@ __global__ void k_mech_integrate(float* __restrict__ soa, double* __restrict__ p
                                  const uint32_t* __restrict__ cell_inst, const CellInst* __restrict__ insts,
                                  float dt_override, const uint8_t* __restrict__ mask)
 {
+    dependents_may_launch();
+    if (!await_predecessors()) return;
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n) return;
     const uint32_t ii = cell_inst[g];
@@ -652,7 +670,7 @@ cudaError_t launch_sec_cell_consts(cudaStream_t st, const float* soa, uint32_t s
 {
     cudaError_t e = cudaMemsetAsync(flags, 0, static_cast<size_t>(n_inst) * sizeof(uint32_t), st);
     if (e != cudaSuccess || n == 0) return e;
-    k_sec_cell_consts<<<blocks_for(n, 256), 256, 0, st>>>(soa, stride, n, cell_inst, insts, rates4, n_rate, dt, cc,
+    launch_chained(st, k_sec_cell_consts, blocks_for(n, 256), 256, 0, soa, stride, n, cell_inst, insts, rates4, n_rate, dt, cc,
                                                            flags);
     return cudaGetLastError();
 }
@@ -662,7 +680,7 @@ cudaError_t launch_sec_permute(cudaStream_t st, const uint32_t* skeys, const uin
                                const uint32_t* flags, const double* cc, uint32_t n_rate, double* cs)
 {
     if (n == 0) return cudaSuccess;
-    k_sec_permute<<<blocks_for(n, 256), 256, 0, st>>>(skeys, sorder, n, cell_inst, insts, invalid_key, flags, cc,
+    launch_chained(st, k_sec_permute, blocks_for(n, 256), 256, 0, skeys, sorder, n, cell_inst, insts, invalid_key, flags, cc,
                                                        n_rate, cs);
     return cudaGetLastError();
 }
@@ -673,7 +691,7 @@ cudaError_t launch_secrete(cudaStream_t st, float* dens, const uint32_t* run_sta
 {
     if (max_runs == 0 || max_s == 0) return cudaSuccess;
     if (block < 32 || block > 256 || block % 32) return cudaErrorInvalidValue;
-    k_secrete<<<blocks_for(max_runs, block), block, 0, st>>>(dens, run_start, run_word, n_runs, insts, cs, cap, flags,
+    launch_chained(st, k_secrete, blocks_for(max_runs, block), block, 0, dens, run_start, run_word, n_runs, insts, cs, cap, flags,
                                                           mask);
     return cudaGetLastError();
 }
@@ -694,7 +712,7 @@ cudaError_t launch_mech_bin(cudaStream_t st, float* soa, uint32_t stride, uint32
 {
     if (n == 0) return cudaSuccess;
     if (block < 32 || block > 1024 || block % 32) return cudaErrorInvalidValue;
-    k_mech_bin<<<blocks_for(n, block), block, 0, st>>>(soa, stride, n, cell_inst, insts, keys, slots, counts, mask);
+    launch_chained(st, k_mech_bin, blocks_for(n, block), block, 0, soa, stride, n, cell_inst, insts, keys, slots, counts, mask);
     return cudaGetLastError();
 }
 
@@ -705,14 +723,14 @@ cudaError_t launch_mech_order(cudaStream_t st, const float* soa, uint32_t stride
 {
     if (n == 0) return cudaSuccess;
     if (block < 32 || block > 1024 || block % 32) return cudaErrorInvalidValue;
-    k_mech_place<<<blocks_for(n, block), block, 0, st>>>(soa, stride, keys, slots, start, n, placed);
+    launch_chained(st, k_mech_place, blocks_for(n, block), block, 0, soa, stride, keys, slots, start, n, placed);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (sorder)
-        k_mech_order<true><<<blocks_for(n, block), block, 0, st>>>(soa, stride, keys, start, placed, n, cell_inst,
+        launch_chained(st, k_mech_order<true>, blocks_for(n, block), block, 0, soa, stride, keys, start, placed, n, cell_inst,
                                                                    reach, sorder, spos, sprm);
     else
-        k_mech_order<false><<<blocks_for(n, block), block, 0, st>>>(soa, stride, keys, start, placed, n, cell_inst,
+        launch_chained(st, k_mech_order<false>, blocks_for(n, block), block, 0, soa, stride, keys, start, placed, n, cell_inst,
                                                                     reach, nullptr, spos, sprm);
     return cudaGetLastError();
 }
@@ -721,7 +739,7 @@ cudaError_t launch_mech_stable_order(cudaStream_t st, const uint32_t* keys, cons
                                      const uint2* placed, uint32_t n, uint32_t* sorder)
 {
     if (n == 0) return cudaSuccess;
-    k_mech_stable_order<<<blocks_for(n, 256), 256, 0, st>>>(keys, start, placed, n, sorder);
+    launch_chained(st, k_mech_stable_order, blocks_for(n, 256), 256, 0, keys, start, placed, n, sorder);
     return cudaGetLastError();
 }
 
@@ -732,7 +750,7 @@ static cudaError_t forces_variant(cudaStream_t st, unsigned grid, int block, con
                                   uint32_t stride, uint32_t* diag_cnt, uint32_t* diag_hash, const uint8_t* mask)
 {
     const size_t smem = static_cast<size_t>(QCAP) * block * sizeof(uint32_t);   // at most 64 KiB
-    k_mech_forces<QCAP, DIAG><<<grid, block, smem, st>>>(spos, sprm, start, n, cell_inst, insts, reach, soa, stride,
+    launch_chained(st, k_mech_forces<QCAP, DIAG>, grid, block, smem, spos, sprm, start, n, cell_inst, insts, reach, soa, stride,
                                                          diag_cnt, diag_hash, mask);
     return cudaGetLastError();
 }
@@ -778,7 +796,7 @@ cudaError_t launch_mech_integrate(cudaStream_t st, float* soa, double* pos64, ui
 {
     if (n == 0) return cudaSuccess;
     if (block < 32 || block > 1024 || block % 32) return cudaErrorInvalidValue;
-    k_mech_integrate<<<blocks_for(n, block), block, 0, st>>>(soa, pos64, stride, n, cell_inst, insts, dt_override,
+    launch_chained(st, k_mech_integrate, blocks_for(n, block), block, 0, soa, pos64, stride, n, cell_inst, insts, dt_override,
                                                              mask);
     return cudaGetLastError();
 }

@@ -488,6 +488,8 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tma(const SweepTile* __restric
                                                    int stage_floats, int nstages, int tab_area, int apply_faces,
                                                    const uint8_t* __restrict__ mask, unsigned* __restrict__ status)
 {
+    dependents_may_launch();
+    if (!await_predecessors()) return;
     // stage: [tile data][tab_area floats of coefficient table]
     extern __shared__ __align__(128) unsigned char smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
@@ -613,9 +615,11 @@ __global__ void __launch_bounds__(256, 3)
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem);
     float* pl = reinterpret_cast<float*>(smem + 128);
+    dependents_may_launch();
+    // the job, the tables and the tensor maps are written once, before any
+    // step; the density and the mask may be the predecessor's
     const PlaneJob jb = jobs[blockIdx.x];
     const uint32_t ii = jb.inst & kPlaneInstMask;
-    if (mask && !(mask[ii] & STEP_DIFFUSE)) return;   // the whole CTA leaves together
     const uint32_t nx = jb.nx, ny = jb.ny, P = plane_pitch(nx, ZK);
     float* tx = pl + plane_data_floats(nx, ny, ZK);
     float* ty = ZK ? tx : tx + tab_floats(nx);
@@ -623,7 +627,10 @@ __global__ void __launch_bounds__(256, 3)
     if (threadIdx.x == 0) {
         mbar_init(bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
     }
+    if (!await_predecessors()) return;
+    if (mask && !(mask[ii] & STEP_DIFFUSE)) return;   // the whole CTA leaves together
     __syncthreads();
     if (threadIdx.x == 0) {
         const uint32_t tbx = ZK ? 0u : tab_floats(nx) * 4u, tby = tab_floats(ny) * 4u;
@@ -763,6 +770,8 @@ __global__ void __launch_bounds__(32 * kLongLines) k_sweep_long(float* __restric
                                                                 const float* __restrict__ tab, int apply_faces,
                                                                 const uint8_t* __restrict__ mask)
 {
+    dependents_may_launch();
+    if (!await_predecessors()) return;
     constexpr int kSeg = 32 * K, kStride = long_stride<K>();
     extern __shared__ float sh[];
     float* sg = sh + kLongLines * kStride;   // g of the segment's positions
@@ -857,6 +866,8 @@ __global__ void __launch_bounds__(32 * kLongLines) k_sweep_long(float* __restric
 
 __global__ void k_dirichlet(float* __restrict__ dens, const FaceJob* __restrict__ jobs)
 {
+    dependents_may_launch();
+    if (!await_predecessors()) return;
     const FaceJob jb = jobs[blockIdx.x];
     float* base = dens + jb.base;
     const uint32_t nx = jb.nx, ny = jb.ny, nz = jb.nz;
@@ -961,11 +972,11 @@ cudaError_t launch_sweep_tma(cudaStream_t st, bool rows, const SweepTile* tiles,
         return cudaErrorInvalidValue;
     const size_t smem = sweep_tma_smem(cfg.warps, cfg.stages, cfg.stage_floats);
     if (rows)
-        k_sweep_tma<true><<<cfg.grid, cfg.warps * 32, smem, st>>>(tiles, ntiles, tab, tmaps,
+        launch_chained(st, k_sweep_tma<true>, cfg.grid, cfg.warps * 32, smem, tiles, ntiles, tab, tmaps,
                                                                    cfg.stage_floats, cfg.stages, cfg.tab_floats,
                                                                    apply_faces, mask, status);
     else
-        k_sweep_tma<false><<<cfg.grid, cfg.warps * 32, smem, st>>>(tiles, ntiles, tab, tmaps,
+        launch_chained(st, k_sweep_tma<false>, cfg.grid, cfg.warps * 32, smem, tiles, ntiles, tab, tmaps,
                                                                     cfg.stage_floats, cfg.stages, cfg.tab_floats,
                                                                     apply_faces, mask, status);
     return cudaGetLastError();
@@ -1096,9 +1107,8 @@ cudaError_t launch_sweep_planes(cudaStream_t st, bool z, int threads, const Plan
                                 const uint8_t* mask, unsigned* status, uint32_t ahead)
 {
     if (njobs == 0) return cudaSuccess;
-    if (z) k_sweep_planes<true><<<njobs, threads, sweep_planes_smem(floats), st>>>(jobs, tab, tmaps, apply_faces, mask, status, ahead);
-    else k_sweep_planes<false><<<njobs, threads, sweep_planes_smem(floats), st>>>(jobs, tab, tmaps, apply_faces, mask, status, ahead);
-    return cudaGetLastError();
+    return launch_chained(st, z ? k_sweep_planes<true> : k_sweep_planes<false>, njobs, threads, sweep_planes_smem(floats), jobs,
+                          tab, tmaps, apply_faces, mask, status, ahead);
 }
 
 template <int K>
@@ -1106,7 +1116,7 @@ static cudaError_t long_variant(cudaStream_t st, float* dens, const SweepTile* t
                                 int apply_faces, const uint8_t* mask)
 {
     const size_t smem = static_cast<size_t>(kLongLines + 2) * long_stride<K>() * sizeof(float);   // at most 43 KB
-    k_sweep_long<K><<<ntiles, 32 * kLongLines, smem, st>>>(dens, tiles, tab, apply_faces, mask);
+    launch_chained(st, k_sweep_long<K>, ntiles, 32 * kLongLines, smem, dens, tiles, tab, apply_faces, mask);
     return cudaGetLastError();
 }
 
@@ -1126,7 +1136,7 @@ cudaError_t launch_sweep_long(cudaStream_t st, float* dens, const SweepTile* til
 cudaError_t launch_dirichlet(cudaStream_t st, float* dens, const FaceJob* jobs, uint32_t njobs)
 {
     if (njobs == 0) return cudaSuccess;
-    k_dirichlet<<<njobs, 256, 0, st>>>(dens, jobs);
+    launch_chained(st, k_dirichlet, njobs, 256, 0, dens, jobs);
     return cudaGetLastError();
 }
 

@@ -105,6 +105,8 @@ __device__ __forceinline__ double norm3(double x, double y, double z)
 __global__ void k_motility(float* __restrict__ soa, uint32_t stride, MotState m, DensView dv, bool have_density,
                            double dt, uint64_t seed, uint64_t step, int layout)
 {
+    dependents_may_launch();
+    if (!await_predecessors()) return;
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m.n) return;
     if (__float_as_uint(soa[static_cast<size_t>(F_IS_ALIVE) * stride + i]) == 0u) return;
@@ -314,9 +316,8 @@ pcg_status pcg_motility_update(pcg_motility* m, pcg_cells* cells, const pcg_me* 
                 m->is_motile.as<uint32_t>(), m->restrict_2d.as<uint32_t>(), m->chem_index.as<int32_t>(),
                 m->chem_dir.as<int32_t>(), m->n_sens ? m->sens.as<double>() : nullptr, m->n_sens, m->n};
     const unsigned grid = (m->n + 127) / 128;
-    k_motility<<<grid, 128, 0, ctx->stream>>>(cells->c.soa.as<float>(), cells->c.max_cells, ms, dv, have, dt, seed,
-                                              step, layout);
-    PCG_CU(ctx, cudaGetLastError());
+    PCG_CU(ctx, launch_chained(ctx->stream, k_motility, grid, 128, 0, cells->c.soa.as<float>(), cells->c.max_cells, ms, dv,
+                               have, dt, seed, step, layout));
     ctx->launches++;
     return PCG_OK;
 }

@@ -151,6 +151,54 @@ enum : uint32_t { INST_REFRESH_VOXELS = 1u };
 // instance takes this diffusion step, bit 1 = it takes this mechanics step.
 enum : uint8_t { STEP_DIFFUSE = 1u, STEP_MECH = 2u };
 
+// ---------------------------------------------------------------- dependent launches
+//
+// A step is a chain of short kernels, and between two of them the GPU idles
+// for 1-2 us (drain, launch, block start-up).  Every kernel of the chains is
+// launched with programmatic stream serialisation: once all blocks of its
+// predecessor have started (dependents_may_launch at their first statement)
+// its blocks take free slots, run what does not depend on the predecessor,
+// and wait (await_predecessors) until it has completed and its writes are
+// visible.  Every block of every kernel waits before it returns, so a
+// kernel's completion implies that of all before it.  In front of anything
+// else (a copy, an event wait) the launch orders itself as usual.  One
+// mechanics period of the 50 x 50 simulation 133 -> 82.5 us, a mechanics
+// update of 100k cells 67.8 -> 52.9 us.  Captured launches (a batch's
+// graphs) keep full edges: with parallel branches the waiting blocks take
+// slots from the branches still running (64 3-D instances 3.69 -> 3.90 ms
+// a period with programmatic edges, 256 2-D ones 1.53 -> 1.69).
+__device__ __forceinline__ void dependents_may_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// False never (a grid has at least one block in z); the branch on it keeps
+// loads of const __restrict__ data, which the compiler may otherwise treat
+// as free to move, behind the wait.
+__device__ __forceinline__ bool await_predecessors()
+{
+    unsigned z;
+    asm volatile("griddepcontrol.wait;\n mov.u32 %0, %%nctaid.z;" : "=r"(z)::"memory");
+    return z != 0;
+}
+
+template <class... KArgs, class... Args>
+cudaError_t launch_chained(cudaStream_t st, void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem,
+                           Args... args)
+{
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+    const cudaError_t e = cudaStreamIsCapturing(st, &cs);
+    if (e != cudaSuccess) return e;
+    cfg.numAttrs = cs == cudaStreamCaptureStatusNone ? 1 : 0;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
 // ---------------------------------------------------------------- launchers
 // All launchers enqueue on 'st' and return the CUDA launch status.
 

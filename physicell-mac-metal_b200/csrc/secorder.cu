@@ -62,6 +62,8 @@ __global__ void __launch_bounds__(kThreads) k_so_hist(const SegTile* __restrict_
                                                       const uint8_t* __restrict__ active, uint32_t* __restrict__ keys,
                                                       int shift, uint32_t R, uint32_t* __restrict__ hist)
 {
+    dependents_may_launch();
+    if (!await_predecessors()) return;
     __shared__ uint32_t cnt[kMaxBins];
     const SegTile tl = tiles[blockIdx.x];
     for (uint32_t d = threadIdx.x; d <= R; d += kThreads) cnt[d] = 0;
@@ -103,6 +105,8 @@ __global__ void __launch_bounds__(kOffThreads, 1) k_so_offsets(const SegTile* __
                                                             const CellInst* __restrict__ insts, uint32_t R,
                                                             uint32_t* __restrict__ hist)
 {
+    dependents_may_launch();
+    if (!await_predecessors()) return;
     __shared__ uint32_t wsum[kOffThreads / 32];
     __shared__ uint32_t rows[kOffSmem / 4];
     const SegTile t0 = tiles[inst_tile[blockIdx.x]];
@@ -192,6 +196,8 @@ __global__ void __launch_bounds__(kThreads) k_so_scatter(const SegTile* __restri
                                                          const double* __restrict__ cc, double* __restrict__ cs,
                                                          uint32_t cap, const uint32_t* __restrict__ flags)
 {
+    dependents_may_launch();
+    if (!await_predecessors()) return;
     __shared__ uint32_t wcnt[kWarps][kMaxBins];
     __shared__ uint32_t cnt[kMaxBins];
     __shared__ uint32_t tbase[kMaxBins];
@@ -327,6 +333,8 @@ __device__ __forceinline__ bool so_head(const uint32_t* __restrict__ skeys, uint
 __global__ void __launch_bounds__(kThreads) k_so_run_count(const uint32_t* __restrict__ skeys, uint32_t n,
                                                            uint32_t* __restrict__ tile_cnt)
 {
+    dependents_may_launch();
+    if (!await_predecessors()) return;
     __shared__ uint32_t ws[kWarps];
     uint32_t c = 0, key;
 #pragma unroll
@@ -351,6 +359,8 @@ __global__ void __launch_bounds__(kThreads) k_so_run_write(const uint32_t* __res
                                                            uint32_t* __restrict__ run_start,
                                                            uint64_t* __restrict__ run_word, uint32_t* __restrict__ n_runs)
 {
+    dependents_may_launch();
+    if (!await_predecessors()) return;
     __shared__ uint32_t wc[kItems * kWarps];   // heads per (row k, warp), then their exclusive scan
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t lt_mask = (1u << lane) - 1u;
@@ -481,15 +491,15 @@ cudaError_t launch_sec_order(cudaStream_t st, const SegTile* tiles, uint32_t nti
         uint32_t* vd = to_out ? sorder : vtmp;
         const int shift = p * digit_bits;
         if (first)
-            k_so_hist<true><<<ntiles, kThreads, 0, st>>>(tiles, soa, stride, insts, active, keys, shift, R, hist);
+            launch_chained(st, k_so_hist<true>, ntiles, kThreads, 0, tiles, soa, stride, insts, active, keys, shift, R, hist);
         else
-            k_so_hist<false><<<ntiles, kThreads, 0, st>>>(tiles, soa, stride, insts, active, const_cast<uint32_t*>(ks),
+            launch_chained(st, k_so_hist<false>, ntiles, kThreads, 0, tiles, soa, stride, insts, active, const_cast<uint32_t*>(ks),
                                                            shift, R, hist);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
-        k_so_offsets<<<n_inst_tiled, kOffThreads, 0, st>>>(tiles, inst_tile, insts, R, hist);
+        launch_chained(st, k_so_offsets, n_inst_tiled, kOffThreads, 0, tiles, inst_tile, insts, R, hist);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
 #define PCG_SO_SCATTER(F, L)                                                                                    \
-    k_so_scatter<F, L><<<ntiles, kThreads, 0, st>>>(tiles, ks, vs, kd, vd, shift, R, hist, insts, invalid_key, cc, cs, \
+    launch_chained(st, k_so_scatter<F, L>, ntiles, kThreads, 0, tiles, ks, vs, kd, vd, shift, R, hist, insts, invalid_key, cc, cs, \
                                                     cap, flags)
         if (first && last) PCG_SO_SCATTER(true, true);
         else if (first) PCG_SO_SCATTER(true, false);
@@ -504,10 +514,10 @@ cudaError_t launch_sec_order(cudaStream_t st, const SegTile* tiles, uint32_t nti
     uint32_t* tile_cnt = static_cast<uint32_t*>(run_scratch);
     uint32_t* tile_off = tile_cnt + ((static_cast<uint64_t>(rt + 1) * sizeof(uint32_t) + 255) / 256) * 256 / sizeof(uint32_t);
     char* rscr = reinterpret_cast<char*>(tile_off) + ((static_cast<uint64_t>(rt + 1) * sizeof(uint32_t) + 255) / 256) * 256;
-    k_so_run_count<<<rt, kThreads, 0, st>>>(skeys, n, tile_cnt);
+    launch_chained(st, k_so_run_count, rt, kThreads, 0, skeys, n, tile_cnt);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if ((e = scan_exclusive(st, tile_cnt, tile_off, rt, rscr)) != cudaSuccess) return e;
-    k_so_run_write<<<rt, kThreads, 0, st>>>(skeys, sorder, n, invalid_key, tile_off, tile_cnt, rt, cell_inst, insts,
+    launch_chained(st, k_so_run_write, rt, kThreads, 0, skeys, sorder, n, invalid_key, tile_off, tile_cnt, rt, cell_inst, insts,
                                              run_start, run_word, n_runs);
     return cudaGetLastError();
 }

@@ -34,6 +34,8 @@ constexpr uint32_t kMask = kRadix - 1;
 __global__ void __launch_bounds__(kThreads) k_radix_hist(const uint32_t* __restrict__ keys, uint32_t n, int shift,
                                                          uint32_t* __restrict__ hist, uint32_t ntiles)
 {
+    dependents_may_launch();
+    if (!await_predecessors()) return;
     __shared__ uint32_t h[kRadix];
     for (int i = threadIdx.x; i < kRadix; i += kThreads) h[i] = 0;
     __syncthreads();
@@ -53,6 +55,8 @@ __global__ void __launch_bounds__(kThreads) k_radix_scatter(const uint32_t* __re
                                                             uint32_t n, int shift,
                                                             const uint32_t* __restrict__ offsets, uint32_t ntiles)
 {
+    dependents_may_launch();
+    if (!await_predecessors()) return;
     __shared__ uint32_t wcnt[kWarps][kRadix];
     __shared__ uint32_t gbase[kRadix];
     __shared__ uint32_t tbase[kRadix];      // first place of each digit in the tile
@@ -134,6 +138,8 @@ __global__ void __launch_bounds__(kThreads) k_radix_scatter(const uint32_t* __re
 __global__ void __launch_bounds__(kThreads) k_tile_sums(const uint32_t* __restrict__ in, uint64_t n,
                                                         uint32_t* __restrict__ sums)
 {
+    dependents_may_launch();
+    if (!await_predecessors()) return;
     __shared__ uint32_t wsum[kWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t base = static_cast<uint64_t>(blockIdx.x) * kTile + static_cast<uint64_t>(threadIdx.x) * kItems;
@@ -194,6 +200,8 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t x, uint32_t* wsum, 
 __global__ void __launch_bounds__(kThreads) k_scan_tiles(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
                                                          uint64_t n, const uint32_t* __restrict__ offs)
 {
+    dependents_may_launch();
+    if (!await_predecessors()) return;
     static_assert(kTile == 2 * 4 * kThreads, "two halves of four values per thread");
     __shared__ uint32_t wsum[kWarps + 1];
     const uint64_t tile = static_cast<uint64_t>(blockIdx.x) * kTile;
@@ -268,17 +276,17 @@ static cudaError_t scan_rec(cudaStream_t st, const uint32_t* in, uint32_t* out, 
     const uint64_t nt = tiles_of(n);
     if (nt == 0) return cudaSuccess;
     if (nt == 1) {
-        k_scan_tiles<<<1, kThreads, 0, st>>>(in, out, n, nullptr);
+        launch_chained(st, k_scan_tiles, 1, kThreads, 0, in, out, n, nullptr);
         return cudaGetLastError();
     }
     uint32_t* sums = reinterpret_cast<uint32_t*>(scratch);
     char* next = scratch + ((nt * sizeof(uint32_t) + 255) / 256) * 256;
-    k_tile_sums<<<static_cast<unsigned>(nt), kThreads, 0, st>>>(in, n, sums);
+    launch_chained(st, k_tile_sums, static_cast<unsigned>(nt), kThreads, 0, in, n, sums);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     e = scan_rec(st, sums, sums, nt, next);
     if (e != cudaSuccess) return e;
-    k_scan_tiles<<<static_cast<unsigned>(nt), kThreads, 0, st>>>(in, out, n, sums);
+    launch_chained(st, k_scan_tiles, static_cast<unsigned>(nt), kThreads, 0, in, out, n, sums);
     return cudaGetLastError();
 }
 
@@ -330,12 +338,12 @@ cudaError_t radix_sort_pairs(cudaStream_t st, const uint32_t* k_in, const uint32
         uint32_t* kd = to_out ? k_out : k_tmp;
         uint32_t* vd = to_out ? v_out : v_tmp;
         const int shift = p * kDigitBits;
-        k_radix_hist<<<nt, kThreads, 0, st>>>(ks, n, shift, hist, nt);
+        launch_chained(st, k_radix_hist, nt, kThreads, 0, ks, n, shift, hist, nt);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         e = scan_exclusive(st, hist, hist, static_cast<uint64_t>(nt) * kRadix, sscr);
         if (e != cudaSuccess) return e;
-        k_radix_scatter<<<nt, kThreads, 0, st>>>(ks, vs, kd, vd, n, shift, hist, nt);
+        launch_chained(st, k_radix_scatter, nt, kThreads, 0, ks, vs, kd, vd, n, shift, hist, nt);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         ks = kd;
