@@ -18,6 +18,12 @@ thread_local std::string g_create_err;
 
 int bad(pcg_ctx* ctx, const char* msg) { return fail(ctx, PCG_ERR_INVALID, msg); }
 
+// Most cells of a single 2-D simulation whose secretion runs inside its
+// plane's CTAs (pcg_me_step): they share S SMs there, the whole GPU in a
+// launch of their own.  10 sub-steps of 50 x 50: 25.5 us fused against 65.5
+// at 500 cells, 73.1 against 71.9 at 5000.
+constexpr uint32_t kFusedStepCells = 4096;
+
 bool same_bytes(const void* a, const void* b, size_t n) { return std::memcmp(a, b, n) == 0; }
 
 // Attach the diffusion grid of 'me' to the single instance of 'cells'.
@@ -279,6 +285,7 @@ pcg_status pcg_me_download(pcg_me* me, float* host, size_t n)
 pcg_status pcg_me_diffuse(pcg_me* me, int n_steps)
 {
     if (!me || n_steps < 0) return PCG_ERR_INVALID;
+    if (me->d.takes_steps(n_steps)) return me->d.steps_2d(n_steps, false, RunArgs{}, 0);
     for (int s = 0; s < n_steps; ++s) PCG_TRY(me->d.sweeps(false, nullptr));
     return PCG_OK;
 }
@@ -309,6 +316,11 @@ pcg_status pcg_me_step(pcg_me* me, pcg_cells* cells, int n_steps)
         PCG_TRY(bind_me(cells, me));
     }
     const double dt = me->d.inst[0].g.dt;
+    if (me->d.takes_steps(n_steps) && (!sec || (cells->c.n <= kFusedStepCells && me->d.steps_fit(cells->c.n)))) {
+        // a 2-D plane: all sub-steps in one launch
+        if (sec) PCG_TRY(cells->c.prepare_secretion(dt, me->d.total_vox));
+        return me->d.steps_2d(n_steps, true, sec ? cells->c.run_args() : RunArgs{}, sec ? cells->c.n : 0);
+    }
     for (int s = 0; s < n_steps; ++s) {
         PCG_TRY(me->d.sweeps(true, nullptr));
         if (sec) {

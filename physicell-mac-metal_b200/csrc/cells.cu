@@ -15,7 +15,7 @@
 // that order; the mechanics binning is a counting sort whose
 // order within a voxel is fixed by ranks (index, and x for the force
 // pass), so every cell's neighbour walk and sum have a fixed order.
-#include "pcg_kernels.cuh"
+#include "secrete.cuh"
 
 namespace pcg {
 
@@ -103,25 +103,6 @@ __global__ void k_sec_permute(const uint32_t* __restrict__ skeys, const uint32_t
         if (f & 2u) cs[n_rate + dst + s] = cc[n_rate + src + s];
         cs[2ull * n_rate + dst + s] = cc[2ull * n_rate + src + s];
     }
-}
-
-// One cell's processSecretion on one substrate (cell_phenotype.cpp:526-564):
-// rho += c0; rho = (rho + c1) / c2; clamp at 0; FP32 store.  A term the
-// instance never has (flags) is exactly +0 and is added as the constant.
-__device__ __forceinline__ float secrete_terms(float rho32, double c0, double c1, double c2)
-{
-    double rho = static_cast<double>(rho32);
-    rho = __dadd_rn(rho, c0);
-    rho = __dadd_rn(rho, c1);
-    rho = __ddiv_rn(rho, c2);
-    if (rho < 0.0) rho = 0.0;
-    return __double2float_rn(rho);
-}
-
-__device__ __forceinline__ float secrete_cell(float rho32, const double* __restrict__ cs, uint64_t o, uint64_t cap,
-                                              uint32_t f)
-{
-    return secrete_terms(rho32, (f & 1u) ? cs[o] : 0.0, (f & 2u) ? cs[cap + o] : 0.0, cs[2 * cap + o]);
 }
 
 // One thread per run: applies the run's cells to its voxel in ascending

@@ -219,7 +219,8 @@ struct PlaneJob {
     uint32_t tab_x, tab_y;   // table offsets (floats)
     float fold_x, T_x, fold_y, T_y;
     uint32_t inst;           // instance | kPlaneDirX | kPlaneDirY | kPlaneFaces | kPlaneZ | kPlaneSlabFace
-    uint32_t _pad[5];
+    uint32_t sub;            // substrate
+    uint32_t _pad[4];
 };
 static_assert(sizeof(PlaneJob) == 64, "PlaneJob is 64 bytes");
 constexpr uint32_t kPlaneDirX = 1u << 31, kPlaneDirY = 1u << 30, kPlaneFaces = 1u << 29;
@@ -245,6 +246,37 @@ __host__ __device__ constexpr uint32_t plane_floats(uint32_t nx, uint32_t ny, bo
 {
     return plane_data_floats(nx, ny, z) + (z ? 0u : tab_floats(nx)) + tab_floats(ny);
 }
+
+// Several sub-steps of 2-D planes in one launch (k_steps_2d), one CTA per
+// plane job of an x-y plane; 'floats' = the largest plane_floats of the jobs.
+// cls: the most chunks of a half line that stay in registers (8: planes of
+// sides up to 64, 16: up to 128, two lanes per line; 0: any, one thread per
+// line in shared memory).  Secretion reads the run list of the secretion
+// order; run_word null: none.
+struct RunArgs {
+    const uint32_t* run_start = nullptr;
+    const uint64_t* run_word = nullptr;
+    const uint32_t* n_runs = nullptr;
+    const uint32_t* inst_run = nullptr;
+    const CellInst* insts = nullptr;
+    const double* cs = nullptr;
+    uint64_t cap = 0;
+    const uint32_t* flags = nullptr;
+};
+constexpr int steps2d_class(uint32_t side) { return side <= 64u ? 8 : side <= 128u ? 16 : 0; }
+// Lines take 16 lines a warp (two lanes each) or 32; the cells' chains want
+// all the warps that the registers of the solve leave.
+constexpr int kSteps2dThreads = 512;
+// Shared memory of a plane with the runs and terms (c2, 1 / c2, c0, c1) of
+// stage_cells cells staged beside it (0: no secretion).
+constexpr int kStageTerms = 4;
+size_t steps2d_smem(uint32_t floats, uint32_t stage_cells);
+cudaError_t steps2d_prepare(int cls);   // opt-in shared memory of a kernel (outside stream capture)
+cudaError_t launch_steps2d(cudaStream_t st, int cls, const PlaneJob* jobs, uint32_t njobs, const float* tab,
+                           const void* tmaps, uint32_t floats, const RunArgs& a, int n_steps, int apply_faces,
+                           uint32_t stage_cells, unsigned* status);
+// Lets a kernel take a CTA's opt-in shared memory (current device).
+cudaError_t allow_max_smem(const void* kernel);
 
 struct TmaCfg { int warps; int stages; int stage_floats; int grid; int tab_floats; };
 
@@ -397,7 +429,8 @@ int so_launches(uint32_t ntiles, int passes, uint32_t n);
 size_t so_run_scratch_bytes(uint32_t max_cells);
 // Keys, the sort and the run list in one call.  Outputs: skeys (global
 // voxel key vox_base + index, or invalid_key) and sorder (cell) per sorted
-// position; *n_runs; run_start (n + 1) and run_word per run.  keys, ktmp
+// position; *n_runs; run_start (n + 1) and run_word per run; inst_run per
+// instance with secreting cells, its first run.  keys, ktmp
 // and vtmp are n-entry work arrays;
 // scratch: so_scratch_bytes, run_scratch: so_run_scratch_bytes; inst_tile:
 // the n_inst_tiled entries of so_tiles.  With cc non-null the last pass
@@ -408,7 +441,7 @@ cudaError_t launch_sec_order(cudaStream_t st, const SegTile* tiles, uint32_t nti
                              int digit_bits, const float* soa, uint32_t stride, const CellInst* insts,
                              const uint8_t* active, const uint32_t* cell_inst, uint32_t invalid_key, uint32_t* keys,
                              uint32_t* ktmp, uint32_t* vtmp, uint32_t* skeys, uint32_t* sorder, void* scratch,
-                             uint32_t* n_runs, uint32_t* run_start, uint64_t* run_word, void* run_scratch,
+                             uint32_t* n_runs, uint32_t* run_start, uint64_t* run_word, uint32_t* inst_run, void* run_scratch,
                              const double* cc, double* cs, uint32_t cap, const uint32_t* flags);
 
 // Radix sort of (key, value) pairs, stable, 'bits' significant key bits.

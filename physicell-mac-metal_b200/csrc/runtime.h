@@ -173,6 +173,14 @@ struct PlaneList {
     uint64_t units = 0;        // voxel-substrates covered
 };
 
+// 2-D planes that take several sub-steps in one launch (k_steps_2d).
+struct StepList {
+    DevBuf jobs;
+    uint32_t n = 0;
+    int cls = 0;               // steps2d_class
+    uint32_t floats = 0;       // largest plane_floats of the jobs
+};
+
 struct SweepList {
     int kind = 0;              // 0 row tiles (TMA), 1 column tiles (TMA), 2 any length (one warp per line)
     int nmax = 0;
@@ -201,6 +209,8 @@ public:
     // x-z plane (zplanes); rest[2] holds the z tiles of the others.
     std::vector<PlaneList> zplanes;
     std::vector<SweepList> rest[3];
+    // A single 2-D simulation's planes again, for steps_2d().
+    std::vector<StepList> steps;
     bool use_planes = true;            // set before build()
     std::string shapes;
 
@@ -212,6 +222,14 @@ public:
     int pin(int kind, int param);                  // one shape for every TMA list of a kind (0 x, 1 columns)
     int sweep(int axis, bool fuse_faces, const uint8_t* mask);
     int sweeps(bool fuse_faces, const uint8_t* mask);
+    // n sub-steps (sweeps, with faces the Dirichlet reset, with run_word the
+    // secretion) of every instance in 'steps'; side streams as launch_planes
+    // stage_cells: the most cells of an instance, whose runs and terms are
+    // staged in shared memory (steps_fit; 0 without secretion)
+    int steps_2d(int n, bool faces, const RunArgs& runs, uint32_t stage_cells);
+    bool steps_fit(uint32_t stage_cells) const;   // they fit beside every plane
+    // one launch of steps_2d is the way to take n sub-steps of every instance
+    bool takes_steps(int n) const;
     int dirichlet();
     int gradients(float* gx, float* gy, float* gz);   // device arrays of total_vox_sub floats, dense per instance
     int upload(uint32_t i, const float* host, bool async_pinned = false);
@@ -240,6 +258,7 @@ private:
     uint32_t cls_floats_[2][kPlaneClasses] = {};
     int cls_threads_[2][kPlaneClasses] = {};
     uint64_t cls_units_[2][kPlaneClasses] = {};
+    int build_steps();
     std::vector<uint8_t> plane_inst_;    // instance's x + y sweeps run as planes
     std::vector<uint8_t> zplane_inst_;   // instance's z sweep runs as x-z planes
     int launch_planes(const std::vector<PlaneList>& pls, bool fuse_faces, const uint8_t* mask);
@@ -285,6 +304,7 @@ public:
     // (rebuilt with the instance table), so_passes x so_bits the digits.
     DevBuf keys, vals, skeys, sorder, ktmp, vtmp, sort_scr, run_scr, tiles, inst_tile;
     DevBuf run_word;   // per run: instance and density element of its voxel (make_run_word)
+    DevBuf inst_run;   // per instance with secreting cells: its first run
     uint32_t invalid_key = 0;
     uint32_t ntiles = 0, max_tiles = 0, n_inst_tiled = 0;
     int so_passes = 1, so_bits = 0;
@@ -314,6 +334,7 @@ public:
     int build_order(uint64_t total_vox);   // order, runs and (once a dt is known) the constants
     int sorted_constants();   // cell-order constants when stale, then their permutation
     int secrete(Diffusion& d, const uint8_t* mask);
+    RunArgs run_args() const;                      // the run list, for steps_2d
     uint64_t device_bytes() const;
 };
 
