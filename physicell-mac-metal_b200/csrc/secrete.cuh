@@ -39,6 +39,39 @@ __device__ __forceinline__ double quotient(double a, double b, double y, bool& o
     return q;
 }
 
+// RN(1 / b) by Newton iterations from the hardware's approximate reciprocal
+// (20 bits, 40, then the full width, then the last place), for b in
+// quotient()'s range.
+__device__ __forceinline__ double reciprocal(double b)
+{
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+#pragma unroll
+    for (int i = 0; i < 3; ++i) y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+    return y;
+}
+
+// Uptake alone (both other terms +0) of one cell on N substrates of a voxel,
+// side by side; rho + 0 + 0 is rho + 0.
+template <int N>
+__device__ __forceinline__ void take_up(float (&rho)[N], const double (&c2)[N])
+{
+    float v[N];
+    bool ok = true;
+#pragma unroll
+    for (int u = 0; u < N; ++u) {
+        double q = quotient(__dadd_rn(static_cast<double>(rho[u]), 0.0), c2[u], reciprocal(c2[u]), ok);
+        if (q < 0.0) q = 0.0;
+        v[u] = __double2float_rn(q);
+    }
+    if (!ok) {
+#pragma unroll
+        for (int u = 0; u < N; ++u) v[u] = secrete_terms(rho[u], 0.0, 0.0, c2[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < N; ++u) rho[u] = v[u];
+}
+
 // One cell on each of B voxels, side by side (y = RN(1 / c2)); a lane whose
 // operands leave quotient()'s range takes the plain division.
 template <int B>
