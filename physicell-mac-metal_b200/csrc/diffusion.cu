@@ -273,6 +273,7 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tma(const SweepTile* __restric
 // SM overlap one plane's copies with another's solves, and each CTA
 // prefetches into L2 (a tensor-box prefetch, no shared memory) the plane of
 // the CTA 'ahead' jobs later, so that CTA's load is served from L2.
+// Large x-z planes come in strips of columns (z lines are independent).
 //
 // What bounds it: the x + y pass by the shared-memory wavefronts of its two
 // solves beside HBM, the z pass by HBM.  Per chunk of a warp's lines a solve
@@ -297,8 +298,8 @@ __global__ void __launch_bounds__(256, 3)
     // step; the density and the mask may be the predecessor's
     const PlaneJob jb = jobs[blockIdx.x];
     const uint32_t ii = jb.inst & kPlaneInstMask;
-    const uint32_t nx = jb.nx, ny = jb.ny, P = plane_pitch(nx, ZK);
-    float* tx = pl + plane_data_floats(nx, ny, ZK);
+    const uint32_t nx = jb.nx, ny = jb.ny, P = ZK ? jb.pitch : plane_pitch(nx, false);
+    float* tx = pl + plane_data_floats(ZK ? P : nx, ny, ZK);
     float* ty = ZK ? tx : tx + tab_floats(nx);
     const void* map = static_cast<const unsigned char*>(tmaps) + static_cast<size_t>(jb.map) * 128;
     if (threadIdx.x == 0) {
@@ -313,7 +314,7 @@ __global__ void __launch_bounds__(256, 3)
         const uint32_t tbx = ZK ? 0u : tab_floats(nx) * 4u, tby = tab_floats(ny) * 4u;
         mbar_arrive_expect_tx(bar, P * ny * 4u + tbx + tby);   // the whole box, fill included
         if (ZK) {
-            tensor_load3(pl, map, 0, static_cast<int>(jb.row0), 0, bar);
+            tensor_load3(pl, map, static_cast<int>(jb.x0), static_cast<int>(jb.row0), 0, bar);
         } else {
             tensor_load2(pl, map, 0, static_cast<int>(jb.row0), bar);
             bulk_load(tx, tab + jb.tab_x, tbx, bar);
@@ -326,7 +327,7 @@ __global__ void __launch_bounds__(256, 3)
             const PlaneJob nj = jobs[blockIdx.x + ahead];
             if (!mask || (mask[nj.inst & kPlaneInstMask] & STEP_DIFFUSE)) {
                 const void* nmap = static_cast<const unsigned char*>(tmaps) + static_cast<size_t>(nj.map) * 128;
-                if (ZK) tensor_prefetch3(nmap, 0, static_cast<int>(nj.row0), 0);
+                if (ZK) tensor_prefetch3(nmap, static_cast<int>(nj.x0), static_cast<int>(nj.row0), 0);
                 else tensor_prefetch2(nmap, 0, static_cast<int>(nj.row0));
             }
         }
@@ -365,14 +366,19 @@ __global__ void __launch_bounds__(256, 3)
         for (uint32_t c = threadIdx.x; c < nx; c += blockDim.x) plane_col(pl + c, static_cast<int>(P), ry, ty);
     if (faces) {
         __syncthreads();
-        const uint32_t step = slab_face ? 1u : (nx > 1 ? nx - 1 : 1u);   // every column, or the first and the last
-        for (uint32_t j = threadIdx.x; j < ny; j += blockDim.x)
-            for (uint32_t c = 0; c < nx; c += step) pl[j * P + c] = ry.T;
+        // every column, or the block's first and last where the job has them
+        const uint32_t x0 = ZK ? jb.x0 : 0u, last = (ZK ? jb.full_nx : nx) - 1u - x0;
+        for (uint32_t j = threadIdx.x; j < ny; j += blockDim.x) {
+            if (slab_face)
+                for (uint32_t c = 0; c < nx; ++c) pl[j * P + c] = ry.T;
+            if (x0 == 0) pl[j * P] = ry.T;
+            if (last < nx) pl[j * P + last] = ry.T;
+        }
     }
     fence_async_smem();
     __syncthreads();
     if (threadIdx.x == 0) {
-        if (ZK) tensor_store3(map, 0, static_cast<int>(jb.row0), 0, pl);
+        if (ZK) tensor_store3(map, static_cast<int>(jb.x0), static_cast<int>(jb.row0), 0, pl);
         else tensor_store2(map, 0, static_cast<int>(jb.row0), pl);
         bulk_commit();
         bulk_wait_read<0>();   // shared memory may be released once the store has read it
@@ -730,12 +736,12 @@ bool encode_plane_map(void* map128, float* block, uint32_t nx, uint32_t ny, uint
 }
 
 // x-z planes of one instance-substrate for the z lines: dims (x, y, z), box
-// round4(nx) x 1 x nz (the full x extent, one y, every z).
-bool encode_xz_plane_map(void* map128, float* block, uint32_t nx, uint32_t ny, uint32_t nz, uint32_t px)
+// width x 1 x nz (width columns, a multiple of 4, one y, every z).
+bool encode_xz_plane_map(void* map128, float* block, uint32_t nx, uint32_t ny, uint32_t nz, uint32_t px, uint32_t width)
 {
     PFN_cuTensorMapEncodeTiled_v12000 fn = encode_fn();
-    const uint32_t bx = (nx + 3u) & ~3u;
-    if (!fn || nx == 0 || bx > 256 || nz == 0 || nz > 256 || ny == 0 || (px & 3u) || px < nx ||
+    const uint32_t bx = width;
+    if (!fn || nx == 0 || bx == 0 || (bx & 3u) || bx > 256 || nz == 0 || nz > 256 || ny == 0 || (px & 3u) || px < nx ||
         (reinterpret_cast<uintptr_t>(block) & 15u))
         return false;
     const cuuint64_t row = static_cast<cuuint64_t>(px) * 4u;

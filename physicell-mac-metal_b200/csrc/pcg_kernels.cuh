@@ -209,9 +209,10 @@ cudaError_t launch_chained(cudaStream_t st, void (*kernel)(KArgs...), unsigned g
 // (rows).  x-y jobs (z slab k of one instance-substrate): the plane tensor
 // map (box row_smem_pitch(nx) x ny, slot 1 of the x rule), first row
 // row0 = k * ny, x and y rules: every row, then every column is solved.
-// z jobs (kPlaneZ: the x-z plane y = row0): the 3-D map of slot 3 of the z
-// rule (box round4(nx) x 1 x nz), ny = nz, the z rule in the y fields:
-// every column (a z line) is solved.
+// z jobs (kPlaneZ: the x-z plane y = row0, or a strip of it from x = x0): the
+// 3-D map of slot 3 of the z rule (box pitch x 1 x nz), nx = the strip's
+// columns, ny = nz, the z rule in the y fields: every column (a z line) is
+// solved.
 struct PlaneJob {
     uint32_t map;
     uint32_t row0;
@@ -220,7 +221,8 @@ struct PlaneJob {
     float fold_x, T_x, fold_y, T_y;
     uint32_t inst;           // instance | kPlaneDirX | kPlaneDirY | kPlaneFaces | kPlaneZ | kPlaneSlabFace
     uint32_t sub;            // substrate
-    uint32_t _pad[4];
+    uint32_t x0, pitch, full_nx;   // z jobs: first column, columns of the box, the block's nx
+    uint32_t _pad;
 };
 static_assert(sizeof(PlaneJob) == 64, "PlaneJob is 64 bytes");
 constexpr uint32_t kPlaneDirX = 1u << 31, kPlaneDirY = 1u << 30, kPlaneFaces = 1u << 29;
@@ -302,7 +304,7 @@ size_t sweep_planes_smem(uint32_t floats);
 // sweep_planes_prepare() first.
 int sweep_planes_ctas(bool z, int threads, uint32_t floats);
 bool encode_plane_map(void* map128, float* block, uint32_t nx, uint32_t ny, uint64_t rows, uint32_t px);
-bool encode_xz_plane_map(void* map128, float* block, uint32_t nx, uint32_t ny, uint32_t nz, uint32_t px);
+bool encode_xz_plane_map(void* map128, float* block, uint32_t nx, uint32_t ny, uint32_t nz, uint32_t px, uint32_t width);
 cudaError_t launch_sweep_tma(cudaStream_t st, bool rows, const SweepTile* tiles, uint32_t ntiles,
                              const float* tab, const void* tmaps, int apply_faces,
                              const uint8_t* mask, unsigned* status, TmaCfg cfg);

@@ -519,18 +519,19 @@ int Diffusion::build(pcg_ctx* c, std::vector<DiffInstance> instances)
         }
         // x-z plane maps (slot 3 of each z rule) for the z sweep
         zplane_inst_.assign(inst.size(), 0);
+        choose_strips();
         for (size_t i = 0; use_planes && i < inst.size(); ++i) {
             const DiffInstance& d = inst[i];
             const uint32_t nx = d.g.nx, nz = d.g.nz;
             if (d.ndim() < 3 || d.g.n_substrates == 0 || ((nx + 3u) & ~3u) > 256 || nz > 256 ||
-                sweep_planes_smem(plane_floats(nx, nz, true)) > kPlaneMaxSmem)
+                sweep_planes_smem(plane_floats(zstrip_[i], nz, true)) > kPlaneMaxSmem)
                 continue;
             bool ok = true;
             for (uint32_t s = 0; s < d.g.n_substrates && ok; ++s) {
                 const uint32_t rule = rule_of(i, s, 2);
                 unsigned char* m = maps.data() + static_cast<size_t>(rule) * kMapsPerRule * 128;
                 ok = encode_xz_plane_map(m + 3 * 128, dens.as<float>() + d.dens_off + s * d.pitch, nx, d.g.ny, nz,
-                                         d.px);
+                                         d.px, zstrip_[i]);
             }
             zplane_inst_[i] = ok ? 1 : 0;
         }
@@ -590,6 +591,25 @@ int Diffusion::regroup_planes(int merge)
     PCG_TRY(plane_lists(ctx, true, cls_jobs_[1], cls_floats_[1], cls_threads_[1], cls_units_[1], kPlaneClasses, merge,
                         zplanes));
     return PCG_OK;
+}
+
+// Columns per x-z plane job of each instance.  Where an SM holds few whole
+// planes, strips of them (z lines are independent) overlap copies and solves
+// better and end in a fuller last wave: three strips at 1 or 2 planes an SM
+// (150^3: one simulation with two substrates 16.6 -> 12.6 us, with four 25.3 ->
+// 21.8, 16 fields 78.4 -> 71.4), two at 3 (120^3: 54.8 -> 53.7 us at 12
+// simulations, 16.4 -> 15.6 at 3).  At 4 (100^3) whole planes were best (51.7
+// us, two strips 52.6, three 56.0).
+void Diffusion::choose_strips()
+{
+    zstrip_.assign(inst.size(), 0);
+    for (size_t i = 0; i < inst.size(); ++i) {
+        const pcg_grid_params& g = inst[i].g;
+        const uint32_t whole = (g.nx + 3u) & ~3u;
+        const size_t per_sm = kPlaneMaxSmem / (sweep_planes_smem(plane_floats(whole, g.nz, true)) + 1024);
+        const uint32_t k = per_sm <= 2 ? 3u : per_sm == 3 ? 2u : 1u;
+        zstrip_[i] = ((g.nx + k - 1) / k + 3u) & ~3u;
+    }
 }
 
 // x-y plane jobs (one per z slab of each substrate of each plane instance),
@@ -662,26 +682,30 @@ int Diffusion::build_planes()
             un[c] += d.nvox() * d.g.n_substrates;
         }
         if (zplane_inst_[i]) {
-            const uint32_t pf = plane_floats(nx, nz, true);
-            const int thr = plane_threads(nx);
+            const uint32_t strip = zstrip_[i], pf = plane_floats(strip, nz, true);
+            const int thr = plane_threads(strip);
             const int c = cls(true, thr, pf);
             cls_threads_[1][c] = std::max(cls_threads_[1][c], thr);
             for (uint32_t s = 0; s < d.g.n_substrates; ++s) {
                 const uint32_t rz_i = rule_of(i, s, 2);
                 const LineRule& rz = h_rules_[rz_i];
-                for (uint32_t y = 0; y < ny; ++y) {
-                    PlaneJob j{};
-                    j.map = rz_i * kMapsPerRule + 3;
-                    j.row0 = y;
-                    j.nx = nx;
-                    j.ny = nz;
-                    j.tab_y = rz.tab;
-                    j.fold_y = rz.fold;
-                    j.T_y = rz.T;
-                    j.inst = static_cast<uint32_t>(i) | kPlaneZ | (rz.dir ? (kPlaneDirY | kPlaneFaces) : 0u) |
-                             ((y == 0 || y + 1 == ny) ? kPlaneSlabFace : 0u);
-                    zjobs[c].push_back(j);
-                }
+                for (uint32_t y = 0; y < ny; ++y)
+                    for (uint32_t x0 = 0; x0 < nx; x0 += strip) {
+                        PlaneJob j{};
+                        j.map = rz_i * kMapsPerRule + 3;
+                        j.row0 = y;
+                        j.nx = std::min(strip, nx - x0);
+                        j.ny = nz;
+                        j.x0 = x0;
+                        j.pitch = strip;
+                        j.full_nx = nx;
+                        j.tab_y = rz.tab;
+                        j.fold_y = rz.fold;
+                        j.T_y = rz.T;
+                        j.inst = static_cast<uint32_t>(i) | kPlaneZ | (rz.dir ? (kPlaneDirY | kPlaneFaces) : 0u) |
+                                 ((y == 0 || y + 1 == ny) ? kPlaneSlabFace : 0u);
+                        zjobs[c].push_back(j);
+                    }
             }
             zfl[c] = std::max(zfl[c], pf);
             zun[c] += d.nvox() * d.g.n_substrates;

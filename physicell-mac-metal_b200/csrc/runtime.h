@@ -261,6 +261,8 @@ private:
     int build_steps();
     std::vector<uint8_t> plane_inst_;    // instance's x + y sweeps run as planes
     std::vector<uint8_t> zplane_inst_;   // instance's z sweep runs as x-z planes
+    std::vector<uint32_t> zstrip_;       // columns of its planes' strips (box width)
+    void choose_strips();
     int launch_planes(const std::vector<PlaneList>& pls, bool fuse_faces, const uint8_t* mask);
     int prepare_forks();   // the side streams launch_planes forks to
     bool planes_for(int axis) const { return axis < 2 ? !planes.empty() : !zplanes.empty(); }
