@@ -185,6 +185,7 @@ int Batch::create(pcg_ctx* c, const pcg_instance_desc* descs, uint32_t n, const 
     if (masked) {
         PCG_CU(ctx, mask_d.alloc(n));
         PCG_CU(ctx, cudaMemsetAsync(mask_d.p, STEP_DIFFUSE | STEP_MECH, n, ctx->stream));
+        mask_now.assign(n, STEP_DIFFUSE | STEP_MECH);
     }
     PCG_CU(ctx, cudaStreamSynchronize(ctx->stream));
     if (use_graphs) {
@@ -450,7 +451,16 @@ int Batch::step_masked(const uint8_t* mask_host, bool any_mech)
 {
     if (!masked) return fail(ctx, PCG_ERR_INVALID, "batch was not created for masked steps");
     cudaStream_t st = ctx->stream;
-    PCG_CU(ctx, cudaMemcpyAsync(mask_d.p, mask_host, mask_d.bytes, cudaMemcpyHostToDevice, st));
+    // the device's mask serves while the bits that this sub-step's kernels
+    // read stay the same (the mechanics bits only where it has a mechanics
+    // step): requests in step with one another copy none
+    const uint8_t read = any_mech ? STEP_DIFFUSE | STEP_MECH : STEP_DIFFUSE;
+    bool same = true;
+    for (size_t i = 0; i < mask_now.size(); ++i) same = same && ((mask_now[i] ^ mask_host[i]) & read) == 0;
+    if (!same) {
+        PCG_CU(ctx, cudaMemcpyAsync(mask_d.p, mask_host, mask_d.bytes, cudaMemcpyHostToDevice, st));
+        mask_now.assign(mask_host, mask_host + mask_now.size());
+    }
     if (use_graphs) {
         PCG_CU(ctx, cudaGraphLaunch(any_mech ? g_mech : g_diff, st));
         ctx->launches += any_mech ? launches_mech : launches_diff;

@@ -66,6 +66,7 @@ public:
     // unchanged until the stream reaches this step).
     int step_masked(const uint8_t* mask_host, bool any_mech);
     DevBuf mask_d;
+    std::vector<uint8_t> mask_now;   // mask_d's contents once the stream is through
     bool masked = false;
     // One sub-step for the instances whose mask bits are set (mask on the device).
     int run_step(bool mech, bool timed, const uint8_t* mask);
