@@ -98,10 +98,25 @@ __global__ void k_sec_permute(const uint32_t* __restrict__ skeys, const uint32_t
     const uint32_t f = flags[ii];
     const uint64_t src = in.rate_off + (g - in.cell_off) * in.S;
     const uint64_t dst = in.rate_off + (q - in.cell_off) * in.S;
-    for (uint32_t s = 0; s < in.S; ++s) {
-        if (f & 1u) cs[dst + s] = cc[src + s];
-        if (f & 2u) cs[n_rate + dst + s] = cc[n_rate + src + s];
-        cs[2ull * n_rate + dst + s] = cc[2ull * n_rate + src + s];
+    // two substrates' loads in flight together: each is a round trip to L2
+    const uint32_t S = in.S;
+    for (uint32_t s = 0; s < S; s += 2u) {
+        const bool two = s + 1u < S;
+        double c[3][2];
+#pragma unroll
+        for (uint32_t a = 0; a < 3u; ++a) {
+            if (a < 2u && !(f >> a & 1u)) continue;
+            const uint64_t o = static_cast<uint64_t>(a) * n_rate + src + s;
+            c[a][0] = cc[o];
+            if (two) c[a][1] = cc[o + 1u];
+        }
+#pragma unroll
+        for (uint32_t a = 0; a < 3u; ++a) {
+            if (a < 2u && !(f >> a & 1u)) continue;
+            const uint64_t o = static_cast<uint64_t>(a) * n_rate + dst + s;
+            cs[o] = c[a][0];
+            if (two) cs[o + 1u] = c[a][1];
+        }
     }
 }
 

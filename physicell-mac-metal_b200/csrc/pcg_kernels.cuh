@@ -427,8 +427,9 @@ uint32_t so_max_tiles(uint32_t max_cells, uint32_t n_inst);
 // and the first tile of every instance that has cells.
 void so_tiles(const CellInst* inst, uint32_t n_inst, std::vector<SegTile>& out, std::vector<uint32_t>& inst_tile);
 size_t so_scratch_bytes(uint32_t max_tiles);
-int so_launches(uint32_t ntiles, int passes, uint32_t n);
+int so_launches(uint32_t ntiles, uint32_t n_inst_tiled, int passes, uint32_t n);
 size_t so_run_scratch_bytes(uint32_t max_cells);
+cudaError_t so_prepare();   // once per device, before the first order
 // Keys, the sort and the run list in one call.  Outputs: skeys (global
 // voxel key vox_base + index, or invalid_key) and sorder (cell) per sorted
 // position; *n_runs; run_start (n + 1) and run_word per run; inst_run per

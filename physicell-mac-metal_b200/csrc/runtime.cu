@@ -1360,6 +1360,7 @@ int Cells::create(pcg_ctx* c, uint32_t maxc, uint32_t rate_capacity, uint32_t n_
     PCG_CU(ctx, run_word.alloc((static_cast<size_t>(max_cells) + 1) * sizeof(uint64_t)));
     PCG_CU(ctx, inst_run.alloc(h_inst.size() * sizeof(uint32_t)));
     PCG_CU(ctx, cudaMemsetAsync(inst_run.p, 0, inst_run.bytes, ctx->stream));
+    PCG_CU(ctx, so_prepare());
     max_tiles = so_max_tiles(max_cells, static_cast<uint32_t>(h_inst.size()));
     PCG_CU(ctx, tiles.alloc(static_cast<size_t>(max_tiles) * sizeof(SegTile)));
     PCG_CU(ctx, inst_tile.alloc(h_inst.size() * sizeof(uint32_t)));
@@ -1500,7 +1501,7 @@ int Cells::build_order(uint64_t total_vox)
                                      consts ? coef_cells.as<double>() : nullptr, coef.as<double>(), cap,
                                      coef_flags.as<uint32_t>());
     if (e != cudaSuccess) return cuda_fail(ctx, e, "secretion order");
-    ctx->launches += so_launches(ntiles, so_passes, n);
+    ctx->launches += so_launches(ntiles, n_inst_tiled, so_passes, n);
     order_dirty = false;
     return PCG_OK;
 }
@@ -1519,7 +1520,7 @@ int Cells::cell_constants(uint32_t cap)
 
 int Cells::order_launches() const
 {
-    return so_launches(ntiles, so_passes, n);
+    return so_launches(ntiles, n_inst_tiled, so_passes, n);
 }
 
 int Cells::sorted_constants()

@@ -32,6 +32,9 @@
 //                 invalid key).
 // The run list of the order follows: a run is the cells of one voxel, and
 // each instance's non-secreting cells form one run marked kRunNone.
+//
+// The cells of a single simulation of up to 32768 cells take one launch
+// instead (k_so_cluster).
 #include "pcg_kernels.cuh"
 
 #include <algorithm>
@@ -420,6 +423,268 @@ __global__ void __launch_bounds__(kThreads) k_so_run_write(const uint32_t* __res
     }
 }
 
+// ------------------------------------------------------------------ one simulation's cells in a cluster
+//
+// All passes and the run list of one instance's n <= 8 * 1024 * I cells in
+// one cluster of 8 CTAs: position p of the order sits in CTA p / (1024 I)
+// (in registers during a pass, thread order as in k_so_scatter: each warp
+// 32 I consecutive positions), and a pass moves every (key, cell) to its
+// next position through the peers' shared memory.  A pass is two cluster
+// barriers: digit counts visible to all (by then every CTA has also taken
+// its positions out of shared memory), and all pairs arrived.
+//
+// What bounds it: latency.  At these sizes a launch of the general path runs
+// for 2-3 us with most of the GPU idle and waits for the one before it, and
+// there are 3 per pass and 3 for the runs; here what lies between two passes
+// is a cluster barrier.  A cluster uses 8 SMs, so what is bound by their load
+// units stays out of it (the constants' gather) or is made regular first:
+// pairs go into digit order in the CTA's own shared memory, so that a warp's
+// stores to the peers cover stretches of consecutive places (a pass over 4096
+// pairs a CTA: 9000 -> 3600 cycles).  Order and constants of 8191 cells on
+// 181 x 117 voxels, two passes: 80 -> 26 us; of 30011 on 61 x 47 x 53, three
+// passes: 86 -> 28 (a mechanics period 247 -> 215 and 296 -> 281).  8 CTAs
+// are the portable cluster size; past 32768 cells it would have to loop over
+// tiles on 8 SMs, where the general path fills more of them.
+constexpr uint32_t kClusterCtas = 8, kClusterThreads = 1024, kClusterWarps = kClusterThreads / 32;
+constexpr uint32_t kClusterMaxItems = 4;
+constexpr uint32_t kClusterMaxCells = kClusterCtas * kClusterThreads * kClusterMaxItems;
+
+__device__ __forceinline__ uint32_t peer_smem(const void* p, uint32_t rank)
+{
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                 : "=r"(a)
+                 : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))), "r"(rank));
+    return a;
+}
+__device__ __forceinline__ uint32_t peer_load(uint32_t a)
+{
+    uint32_t v;
+    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void peer_store(uint32_t a, uint32_t v)
+{
+    asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
+}
+__device__ __forceinline__ void peer_store16(uint32_t a, uint32_t v)
+{
+    asm volatile("st.shared::cluster.u16 [%0], %1;" ::"r"(a), "h"(static_cast<uint16_t>(v)) : "memory");
+}
+// every thread of the cluster arrives, release / acquire
+__device__ __forceinline__ void cluster_barrier()
+{
+    asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
+}
+
+// The lanes whose digit (at most R + 1) equals this lane's, by one ballot per
+// bit: independent instructions, where __match_any_sync is a serial one.
+__device__ __forceinline__ uint32_t same_digit(uint32_t d)
+{
+    uint32_t peers = 0xffffffffu;
+#pragma unroll
+    for (int b = 0; b <= kMaxDigitBits; ++b) {
+        const bool one = (d >> b) & 1u;
+        const uint32_t m = __ballot_sync(0xffffffffu, one);
+        peers &= one ? m : ~m;
+    }
+    return peers;
+}
+
+template <uint32_t I>
+struct ClusterSmem {
+    static constexpr uint32_t kOwn = kClusterThreads * I;    // positions of one CTA
+    uint32_t bk[kOwn], sk[kOwn];                             // keys: at their positions; in digit order
+    uint32_t cnt[kMaxBins], tbase[kMaxBins], delta[kMaxBins];
+    uint32_t wsum[kClusterWarps], heads[kClusterCtas];
+    uint16_t bv[kOwn], sv[kOwn];                             // cells (within the instance), beside the keys
+    uint16_t wcnt[kClusterWarps][kMaxBins + 1];              // digit counts per warp, then each warp's first place
+};
+
+template <uint32_t I>
+__global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterThreads)
+    k_so_cluster(const SegTile* __restrict__ tiles, const float* __restrict__ soa, uint32_t stride, uint32_t n, int passes,
+                 int digit_bits, const CellInst* __restrict__ insts, const uint8_t* __restrict__ active,
+                 uint32_t invalid_key, uint32_t* __restrict__ skeys, uint32_t* __restrict__ sorder,
+                 uint32_t* __restrict__ run_start, uint64_t* __restrict__ run_word, uint32_t* __restrict__ n_runs,
+                 uint32_t* __restrict__ inst_run)
+{
+    constexpr uint32_t kOwn = ClusterSmem<I>::kOwn;
+    extern __shared__ __align__(16) unsigned char so_smem[];
+    ClusterSmem<I>& m = *reinterpret_cast<ClusterSmem<I>*>(so_smem);
+    dependents_may_launch();
+    if (!await_predecessors()) return;
+    const uint32_t rank = blockIdx.x;   // one cluster: the block's rank in it
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint32_t lt_mask = (1u << lane) - 1u;
+    const uint32_t R = 1u << digit_bits;
+    const uint32_t ii = tiles[0].inst;
+    const CellInst& in = insts[ii];
+    const uint32_t nv = in.nx * in.ny * in.nz, S = in.S, off = in.cell_off;
+    const uint32_t t0 = warp * 32u * I + lane, p0 = rank * kOwn + t0;   // item r: position p0 + 32 r
+    const uint32_t own = rank * kOwn >= n ? 0u : min(kOwn, n - rank * kOwn);
+    uint32_t kk[I], vv[I];
+#pragma unroll
+    for (uint32_t r = 0; r < I; ++r) {
+        const uint32_t p = p0 + 32u * r;
+        vv[r] = p;
+        kk[r] = kInvalid;
+        if (p < n) {
+            const uint32_t v = __float_as_uint(soa[static_cast<size_t>(F_VOXEL_IDX) * stride + off + p]);
+            if ((active == nullptr || active[off + p] != 0) && v < nv && S > 0) kk[r] = v;
+        }
+    }
+    for (int pass = 0; pass < passes; ++pass) {
+        const int shift = pass * digit_bits;
+        for (uint32_t d = lane; d <= R; d += 32u) m.wcnt[warp][d] = 0;
+        uint32_t rk[I], dg[I], peers[I];
+#pragma unroll
+        for (uint32_t r = 0; r < I; ++r) {
+            dg[r] = p0 + 32u * r < n ? so_digit(kk[r], shift, R) : R + 1u;   // R + 1 marks an empty place
+            peers[r] = same_digit(dg[r]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (uint32_t r = 0; r < I; ++r) {
+            const bool ok = dg[r] <= R;
+            const uint32_t at = ok ? m.wcnt[warp][dg[r]] : 0u;
+            rk[r] = at + __popc(peers[r] & lt_mask);
+            __syncwarp();
+            if (ok && (peers[r] & lt_mask) == 0u) m.wcnt[warp][dg[r]] = static_cast<uint16_t>(at + __popc(peers[r]));
+            __syncwarp();
+        }
+        __syncthreads();
+        uint32_t mine = 0;   // this CTA's count of digit threadIdx.x
+        if (threadIdx.x <= R) {
+            constexpr uint32_t kBatch = 16;
+#pragma unroll
+            for (uint32_t w0 = 0; w0 < kClusterWarps; w0 += kBatch) {
+                uint32_t c[kBatch];
+#pragma unroll
+                for (uint32_t w = 0; w < kBatch; ++w) c[w] = m.wcnt[w0 + w][threadIdx.x];
+#pragma unroll
+                for (uint32_t w = 0; w < kBatch; ++w) {
+                    m.wcnt[w0 + w][threadIdx.x] = static_cast<uint16_t>(mine);
+                    mine += c[w];
+                }
+            }
+            m.cnt[threadIdx.x] = mine;
+        }
+        cluster_barrier();
+        // digits in order over all CTAs, a digit's CTAs in order; one scan
+        // for the cluster's totals (at most 32768) and this CTA's counts
+        uint32_t tot = 0, before = 0;
+        if (threadIdx.x <= R) {
+#pragma unroll
+            for (uint32_t c = 0; c < kClusterCtas; ++c) {
+                const uint32_t v = peer_load(peer_smem(&m.cnt[threadIdx.x], c));
+                tot += v;
+                before += c < rank ? v : 0u;
+            }
+        }
+        const uint32_t both = tot | mine << 16;
+        uint32_t incl = both;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= static_cast<uint32_t>(o)) incl += y;
+        }
+        if (lane == 31u) m.wsum[warp] = incl;
+        __syncthreads();
+        if (threadIdx.x <= R) {
+            uint32_t ex = incl - both;
+            for (uint32_t w = 0; w < warp; ++w) ex += m.wsum[w];
+            m.tbase[threadIdx.x] = ex >> 16;
+            m.delta[threadIdx.x] = before + (ex & 0xffffu) - (ex >> 16);
+        }
+        __syncthreads();
+        // into digit order here first: a warp's stores to the peers then
+        // cover stretches of consecutive places
+#pragma unroll
+        for (uint32_t r = 0; r < I; ++r) {
+            if (dg[r] > R) continue;
+            const uint32_t t = m.tbase[dg[r]] + m.wcnt[warp][dg[r]] + rk[r];
+            m.sk[t] = kk[r];
+            m.sv[t] = static_cast<uint16_t>(vv[r]);
+        }
+        __syncthreads();
+#pragma unroll
+        for (uint32_t r = 0; r < I; ++r) {
+            const uint32_t t = r * kClusterThreads + threadIdx.x;
+            if (t >= own) continue;
+            const uint32_t key = m.sk[t], dst = t + m.delta[so_digit(key, shift, R)];
+            peer_store(peer_smem(&m.bk[dst % kOwn], dst / kOwn), key);
+            peer_store16(peer_smem(&m.bv[dst % kOwn], dst / kOwn), m.sv[t]);
+        }
+        cluster_barrier();
+#pragma unroll
+        for (uint32_t r = 0; r < I; ++r) {
+            kk[r] = m.bk[t0 + 32u * r];   // stale past n, not used
+            vv[r] = m.bv[t0 + 32u * r];
+        }
+    }
+    // run heads: the CTA's count goes to every CTA
+    uint32_t hb = 0, ahead[I], wheads = 0;
+#pragma unroll
+    for (uint32_t r = 0; r < I; ++r) {
+        const uint32_t t = t0 + 32u * r, p = p0 + 32u * r;
+        bool h = p < n;
+        if (h && p > 0) h = (t > 0 ? m.bk[t - 1] : peer_load(peer_smem(&m.bk[kOwn - 1], rank - 1u))) != kk[r];
+        const uint32_t b = __ballot_sync(0xffffffffu, h);
+        hb |= (h ? 1u : 0u) << r;
+        ahead[r] = wheads + __popc(b & lt_mask);
+        wheads += __popc(b);
+    }
+    if (lane == 0) m.wsum[warp] = wheads;
+    __syncthreads();
+    uint32_t first, all;
+    {
+        const uint32_t c = m.wsum[lane];   // as many warps as lanes
+        first = __reduce_add_sync(0xffffffffu, lane < warp ? c : 0u);
+        all = __reduce_add_sync(0xffffffffu, c);
+    }
+    if (threadIdx.x < kClusterCtas) peer_store(peer_smem(&m.heads[rank], threadIdx.x), all);
+    cluster_barrier();   // the last access to a peer lies before it
+    uint32_t total = 0;
+#pragma unroll
+    for (uint32_t c = 0; c < kClusterCtas; ++c) {
+        first += c < rank ? m.heads[c] : 0u;
+        total += m.heads[c];
+    }
+#pragma unroll
+    for (uint32_t r = 0; r < I; ++r) {
+        const uint32_t p = p0 + 32u * r;
+        const bool sec = kk[r] != kInvalid;
+        if (p < n) {
+            skeys[off + p] = sec ? in.vox_base + kk[r] : invalid_key;
+            sorder[off + p] = off + vv[r];
+        }
+        if ((hb >> r) & 1u) {
+            const uint32_t q = first + ahead[r];
+            run_start[q] = off + p;
+            uint64_t elem = 0;
+            if (sec) {
+                const uint32_t row = kk[r] / in.nx;
+                elem = in.dens_off + static_cast<uint64_t>(row) * in.px + (kk[r] - row * in.nx);
+                if (p == 0) inst_run[ii] = q;
+            }
+            run_word[q] = make_run_word(sec ? ii : kRunNone, elem);
+        }
+    }
+    if (rank == 0 && threadIdx.x == 0) {
+        run_start[total] = off + n;
+        *n_runs = total;
+    }
+}
+
+cudaError_t so_prepare()
+{
+    cudaError_t e = allow_max_smem(reinterpret_cast<const void*>(k_so_cluster<1>));
+    if (e == cudaSuccess) e = allow_max_smem(reinterpret_cast<const void*>(k_so_cluster<2>));
+    if (e == cudaSuccess) e = allow_max_smem(reinterpret_cast<const void*>(k_so_cluster<kClusterMaxItems>));
+    return e;
+}
+
 // ------------------------------------------------------------------ host
 
 void so_plan(uint32_t max_local_voxels, int* passes, int* digit_bits)
@@ -466,9 +731,13 @@ size_t so_run_scratch_bytes(uint32_t max_cells)
     return 2 * ((rt * sizeof(uint32_t) + 255) / 256) * 256 + scan_scratch_bytes(rt);
 }
 
-int so_launches(uint32_t ntiles, int passes, uint32_t n)
+// One simulation's cells, as many as a cluster holds.
+static bool takes_cluster(uint32_t n_inst_tiled, uint32_t n) { return n_inst_tiled == 1 && n <= kClusterMaxCells; }
+
+int so_launches(uint32_t ntiles, uint32_t n_inst_tiled, int passes, uint32_t n)
 {
     if (n == 0 || ntiles == 0) return 0;
+    if (takes_cluster(n_inst_tiled, n)) return 2;
     return passes * 3 + 2 + scan_launches(run_tiles(n));
 }
 
@@ -482,6 +751,20 @@ cudaError_t launch_sec_order(cudaStream_t st, const SegTile* tiles, uint32_t nti
 {
     if (n == 0 || ntiles == 0) return cudaSuccess;
     if (digit_bits > kMaxDigitBits || passes < 1) return cudaErrorInvalidValue;
+    if (takes_cluster(n_inst_tiled, n)) {
+        const uint32_t per = (n + kClusterCtas * kClusterThreads - 1) / (kClusterCtas * kClusterThreads);
+        auto run = [&](auto kernel, size_t smem) {
+            return launch_chained(st, kernel, kClusterCtas, kClusterThreads, smem, tiles, soa, stride, n, passes, digit_bits,
+                                  insts, active, invalid_key, skeys, sorder, run_start, run_word, n_runs, inst_run);
+        };
+        const cudaError_t e = per <= 1   ? run(k_so_cluster<1>, sizeof(ClusterSmem<1>))
+                              : per <= 2 ? run(k_so_cluster<2>, sizeof(ClusterSmem<2>))
+                                         : run(k_so_cluster<kClusterMaxItems>, sizeof(ClusterSmem<kClusterMaxItems>));
+        if (e != cudaSuccess || cc == nullptr) return e;
+        // the constants' gather by all SMs: 9 values of 8191 cells take 8
+        // SMs' load units 4 us, a launch 2.5
+        return launch_sec_permute(st, skeys, sorder, n, cell_inst, insts, invalid_key, flags, cc, cap, cs);
+    }
     const uint32_t R = 1u << digit_bits;
     uint32_t* hist = static_cast<uint32_t*>(scratch);
     const uint32_t* ks = keys;
