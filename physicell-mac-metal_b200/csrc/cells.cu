@@ -148,21 +148,72 @@ __device__ __forceinline__ void take_up_run(float* __restrict__ d, uint64_t pitc
     for (int u = 0; u < N; ++u) d[u * pitch] = rho[u];
 }
 
+constexpr int kWideBlock = 128;   // k_secrete<true>: 256 leave a quarter of the registers unused
+
+// All terms of a run's cells on N adjacent substrates, the same way.
+template <int N>
+__device__ __forceinline__ void apply_run(float* __restrict__ d, uint64_t pitch, const double* __restrict__ c, uint64_t cap,
+                                          uint32_t f, uint32_t S, uint32_t len)
+{
+    double c0[N], c1[N], c2[N];
+    float rho[N];
+    auto terms = [&](double (&x)[N], double (&y)[N], double (&z)[N], bool more) {
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            x[u] = more && (f & 1u) ? c[u] : 0.0;
+            y[u] = more && (f & 2u) ? c[cap + u] : 0.0;
+            z[u] = more ? c[2 * cap + u] : 1.0;
+        }
+    };
+    terms(c0, c1, c2, true);
+#pragma unroll
+    for (int u = 0; u < N; ++u) rho[u] = d[u * pitch];
+    for (;;) {
+        double n0[N], n1[N], n2[N], y[N];
+        bool act[N];
+        c += S;
+        const bool more = --len > 0;
+        terms(n0, n1, n2, more);
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            y[u] = reciprocal(c2[u]);
+            act[u] = true;
+        }
+        secrete_side_by_side<N>(rho, c0, c1, c2, y, act);
+        if (!more) break;
+#pragma unroll
+        for (int u = 0; u < N; ++u) {
+            c0[u] = n0[u];
+            c1[u] = n1[u];
+            c2[u] = n2[u];
+        }
+    }
+#pragma unroll
+    for (int u = 0; u < N; ++u) d[u * pitch] = rho[u];
+}
+
 // One thread per run: applies the run's cells to its voxel in ascending
 // cell index (the stable order), FP64 per cell with the FP32 store after
-// each cell.  The run's metadata is read once; with one or two substrates
-// both are held in registers and advanced together.  Constants: three
-// arrays of cap (c0, c1, c2), entry (cell in sorted order, substrate).
+// each cell.  The run's metadata is read once; adjacent substrates are held
+// in registers and advanced together.  Constants: three arrays of cap (c0,
+// c1, c2), entry (cell in sorted order, substrate).
 // What bounds it: the latency of run data, then density and terms (scattered
-// sectors), and in crowded voxels the cells' chain.  So cells that only take
-// up (the common case) advance two substrates side by side with the next
-// cell's terms in flight and the division as quotient() (as a subroutine it
-// takes 128 cycles and overlaps nothing): 2.5 M cells in 256 2-D instances
-// 52.5 -> 40.8 us a sub-step, 3.0 M in 64 3-D ones 56.9 -> 50.9.  Measured and
-// not taken: a thread per run and substrate (96 and 79 us, every thread
-// reads the run's data), the same pipelining for cells with all terms
-// (their registers cost the uptake path an occupancy step).
-__global__ void __launch_bounds__(256, 6) k_secrete(float* __restrict__ dens, const uint32_t* __restrict__ run_start,
+// sectors), and in crowded voxels the cells' chain.  So a thread advances
+// several substrates side by side with the next cell's terms in flight and
+// the division as quotient() (as a subroutine it takes 128 cycles and
+// overlaps nothing).  How many depends on the number of runs:
+//   WIDE (launch_secrete's rule): few runs, at most some waves of the GPU:
+//   each thread's own latency counts, so four substrates that only take up,
+//   three with all terms.  90 registers.  A sub-step of 200000 cells on four
+//   substrates 15.4 -> 11.0 us, of 8191 with all terms on three 7.1 -> 3.8.
+//   else: threads in flight count; two substrates that only take up, 40
+//   registers: 2.5 M cells in 256 2-D instances 52.5 -> 40.8 us a sub-step,
+//   3.0 M in 64 3-D ones 56.9 -> 50.9 (WIDE: a mechanics period 10 and 3 %
+//   longer).
+// Measured and not taken: a thread per run and substrate (96 and 79 us,
+// every thread reads the run's data).
+template <bool WIDE>
+__global__ void __launch_bounds__(WIDE ? kWideBlock : 256, WIDE ? 5 : 6) k_secrete(float* __restrict__ dens, const uint32_t* __restrict__ run_start,
                           const uint64_t* __restrict__ run_word, const uint32_t* __restrict__ n_runs,
                           const CellInst* __restrict__ insts, const double* __restrict__ cs, uint64_t cap,
                           const uint32_t* __restrict__ flags, const uint8_t* __restrict__ mask)
@@ -184,7 +235,24 @@ __global__ void __launch_bounds__(256, 6) k_secrete(float* __restrict__ dens, co
     const uint64_t base = in.rate_off + (p0 - in.cell_off) * in.S;   // 32-bit slots, as the rates
     const uint32_t S = in.S;
     const uint32_t f = flags[ii];
-    if (f == 0) {   // cells that only take up
+    if (WIDE) {
+        const double* c = cs + base;
+        const uint32_t len = p1 - p0;
+        uint32_t s = 0;
+        if (f == 0) {   // cells that only take up
+            c += 2 * cap;
+            for (; s + 3 < S; s += 4, d += 4 * in.sub_pitch) take_up_run<4>(d, in.sub_pitch, c + s, S, len);
+            if (s + 2 < S) take_up_run<3>(d, in.sub_pitch, c + s, S, len);
+            else if (s + 1 < S) take_up_run<2>(d, in.sub_pitch, c + s, S, len);
+            else if (s < S) take_up_run<1>(d, 0, c + s, S, len);
+            return;
+        }
+        for (; s + 2 < S; s += 3, d += 3 * in.sub_pitch) apply_run<3>(d, in.sub_pitch, c + s, cap, f, S, len);
+        if (s + 1 < S) apply_run<2>(d, in.sub_pitch, c + s, cap, f, S, len);
+        else if (s < S) apply_run<1>(d, 0, c + s, cap, f, S, len);
+        return;
+    }
+    if (f == 0) {
         const double* c = cs + 2 * cap + base;
         uint32_t s = 0;
         for (; s + 1 < S; s += 2, d += 2 * in.sub_pitch) take_up_run<2>(d, in.sub_pitch, c + s, S, p1 - p0);
@@ -731,9 +799,19 @@ cudaError_t launch_secrete(cudaStream_t st, float* dens, const uint32_t* run_sta
 {
     if (max_runs == 0 || max_s == 0) return cudaSuccess;
     if (block < 32 || block > 256 || block % 32) return cudaErrorInvalidValue;
-    launch_chained(st, k_secrete, blocks_for(max_runs, block), block, 0, dens, run_start, run_word, n_runs, insts, cs, cap, flags,
-                                                          mask);
-    return cudaGetLastError();
+    // wide up to four waves of the GPU (5 x 128 threads on 148 SMs: 379k
+    // runs), eight from three substrates on, where the other form passes over
+    // the run more than once.  A mechanics period on 100^3 voxels, wide / not:
+    // 400000 cells 333 / 340 us (one substrate), 374 / 414 (two), 570 / 647
+    // (four); 800000 586 / 549, 631 / 626, 942 / 1236
+    constexpr uint32_t kWideRuns = 4u * 148u * 5u * kWideBlock;
+    if (max_runs <= (max_s > 2 ? 2u * kWideRuns : kWideRuns)) {
+        const int wide = std::min(block, kWideBlock);
+        return launch_chained(st, k_secrete<true>, blocks_for(max_runs, wide), wide, 0, dens, run_start, run_word, n_runs,
+                              insts, cs, cap, flags, mask);
+    }
+    return launch_chained(st, k_secrete<false>, blocks_for(max_runs, block), block, 0, dens, run_start, run_word, n_runs, insts,
+                          cs, cap, flags, mask);
 }
 
 cudaError_t launch_cells_move(cudaStream_t st, float* soa, uint32_t stride, const uint2* moves, uint32_t n_moves,
