@@ -20,15 +20,15 @@ namespace {
 
 constexpr uint32_t kStaticMaxPairs = PCG_SORT_STATIC_MAX_PAIRS;
 constexpr size_t kTmpBytes = static_cast<size_t>(kStaticMaxPairs) * sizeof(uint32_t);   // one ping-pong array
-// Per-tile digit histograms and the scan's tile sums for kStaticMaxPairs
-// keys take about 129 KiB; the reservation leaves room and is checked against the
-// sort's own requirement before the first use.
+// Per-tile digit counts for kStaticMaxPairs keys take 128 KiB; the
+// reservation leaves room and is checked against the sort's own requirement
+// before the first use.
 constexpr size_t kHistBytes = 512u << 10;
 constexpr size_t kScratchBytes = 2 * kTmpBytes + kHistBytes;
 
 // The only scratch of pcg_sort_pairs_static (2.5 MiB per device).  Nothing
-// in it has to start at zero: every pass writes the histograms, tile sums
-// and ping-pong keys it later reads.
+// in it has to start at zero: every pass writes the counts and
+// ping-pong keys it later reads.
 static __device__ __align__(256) unsigned char g_sort_scratch[kScratchBytes];
 
 constexpr int kMaxDevices = 64;

@@ -179,6 +179,22 @@ __device__ __forceinline__ bool await_predecessors()
     return z != 0;
 }
 
+// The lanes of the warp whose digit (at most 2^BITS + 1) equals this lane's,
+// by one ballot per bit: independent instructions, where __match_any_sync is
+// a serial one.
+template <int BITS>
+__device__ __forceinline__ uint32_t same_digit(uint32_t d)
+{
+    uint32_t peers = 0xffffffffu;
+#pragma unroll
+    for (int b = 0; b <= BITS; ++b) {
+        const bool one = (d >> b) & 1u;
+        const uint32_t m = __ballot_sync(0xffffffffu, one);
+        peers &= one ? m : ~m;
+    }
+    return peers;
+}
+
 template <class... KArgs, class... Args>
 cudaError_t launch_chained(cudaStream_t st, void (*kernel)(KArgs...), unsigned grid, unsigned block, size_t smem,
                            Args... args)

@@ -24,7 +24,7 @@
 //                 cell_off, then each tile's row turned into the first place
 //                 of each of its digit runs (digit-major, tiles in order)
 //   k_so_scatter  per tile: stable ranks (each warp ranks its 256 keys with
-//                 __match_any_sync and its own running digit counts, warps
+//                 one ballot per digit bit and its own running counts, warps
 //                 combined in order), the tile laid out in shared
 //                 memory in digit order, then written so that consecutive
 //                 threads store consecutive elements of one digit's run; the
@@ -227,13 +227,16 @@ __global__ void __launch_bounds__(kThreads) k_so_scatter(const SegTile* __restri
     __syncthreads();
     // stable ranks within each warp's 256 keys, against the warp's own counts
     const uint32_t lt_mask = (1u << lane) - 1u;
+    uint32_t peers[kItems];
+#pragma unroll
+    for (int r = 0; r < kItems; ++r) peers[r] = same_digit<kMaxDigitBits>(dg[r]);
 #pragma unroll
     for (int r = 0; r < kItems; ++r) {
-        const uint32_t peers = __match_any_sync(0xffffffffu, dg[r]);
         const bool ok = dg[r] <= R;
-        rk[r] = (ok ? wcnt[warp][dg[r]] : 0u) + __popc(peers & lt_mask);
+        const uint32_t at = ok ? wcnt[warp][dg[r]] : 0u;
+        rk[r] = at + __popc(peers[r] & lt_mask);
         __syncwarp();
-        if (ok && lane == __ffs(peers) - 1) wcnt[warp][dg[r]] += __popc(peers);
+        if (ok && (peers[r] & lt_mask) == 0u) wcnt[warp][dg[r]] = at + __popc(peers[r]);
         __syncwarp();
     }
     __syncthreads();
@@ -477,20 +480,6 @@ __device__ __forceinline__ void cluster_barrier()
     asm volatile("barrier.cluster.arrive.release;\n barrier.cluster.wait.acquire;" ::: "memory");
 }
 
-// The lanes whose digit (at most R + 1) equals this lane's, by one ballot per
-// bit: independent instructions, where __match_any_sync is a serial one.
-__device__ __forceinline__ uint32_t same_digit(uint32_t d)
-{
-    uint32_t peers = 0xffffffffu;
-#pragma unroll
-    for (int b = 0; b <= kMaxDigitBits; ++b) {
-        const bool one = (d >> b) & 1u;
-        const uint32_t m = __ballot_sync(0xffffffffu, one);
-        peers &= one ? m : ~m;
-    }
-    return peers;
-}
-
 template <uint32_t I>
 struct ClusterSmem {
     static constexpr uint32_t kOwn = kClusterThreads * I;    // positions of one CTA
@@ -541,7 +530,7 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
 #pragma unroll
         for (uint32_t r = 0; r < I; ++r) {
             dg[r] = p0 + 32u * r < n ? so_digit(kk[r], shift, R) : R + 1u;   // R + 1 marks an empty place
-            peers[r] = same_digit(dg[r]);
+            peers[r] = same_digit<kMaxDigitBits>(dg[r]);
         }
         __syncwarp();
 #pragma unroll
