@@ -445,7 +445,7 @@ void so_tiles(const CellInst* inst, uint32_t n_inst, std::vector<SegTile>& out, 
 size_t so_scratch_bytes(uint32_t max_tiles);
 int so_launches(uint32_t ntiles, uint32_t n_inst_tiled, int passes, uint32_t n);
 size_t so_run_scratch_bytes(uint32_t max_cells);
-cudaError_t so_prepare();   // once per device, before the first order
+cudaError_t so_prepare(uint32_t max_cells);   // before the first order of a store of max_cells
 // Keys, the sort and the run list in one call.  Outputs: skeys (global
 // voxel key vox_base + index, or invalid_key) and sorder (cell) per sorted
 // position; *n_runs; run_start (n + 1) and run_word per run; inst_run per

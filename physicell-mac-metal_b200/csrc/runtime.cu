@@ -721,22 +721,17 @@ int Diffusion::build_planes()
     return prepare_forks();
 }
 
-// The step list of a single 2-D simulation: its planes are one size.
+// The step list of a single 2-D simulation: its planes are one size, so they
+// are one plane list, whose jobs the steps share.
 int Diffusion::build_steps()
 {
     steps.clear();
-    if (inst.size() != 1 || inst[0].ndim() != 2 || !plane_inst_[0]) return PCG_OK;
-    std::vector<PlaneJob> v;
-    for (int c = 0; c < kPlaneClasses; ++c) v.insert(v.end(), cls_jobs_[0][c].begin(), cls_jobs_[0][c].end());
+    if (inst.size() != 1 || inst[0].ndim() != 2 || planes.size() != 1) return PCG_OK;
     steps.emplace_back();
     StepList& l = steps.back();
-    l.n = static_cast<uint32_t>(v.size());
     l.cls = steps2d_class(std::max(inst[0].g.nx, inst[0].g.ny));
     l.floats = plane_floats(inst[0].g.nx, inst[0].g.ny);
     PCG_CU(ctx, steps2d_prepare(l.cls));
-    PCG_CU(ctx, l.jobs.alloc(v.size() * sizeof(PlaneJob)));
-    PCG_CU(ctx, cudaMemcpyAsync(l.jobs.p, v.data(), v.size() * sizeof(PlaneJob), cudaMemcpyHostToDevice, ctx->stream));
-    PCG_CU(ctx, cudaStreamSynchronize(ctx->stream));   // the host vector goes
     return PCG_OK;
 }
 
@@ -1010,7 +1005,7 @@ int Diffusion::steps_2d(int n, bool faces, const RunArgs& runs, uint32_t stage_c
     for (int s = 0; s < n; s += kMaxFusedSteps) {
         const int k = std::min(kMaxFusedSteps, n - s);
         for (const StepList& l : steps) {
-            cudaError_t e = launch_steps2d(ctx->stream, l.cls, l.jobs.as<PlaneJob>(), l.n, tab.as<float>(), tmaps.p,
+            cudaError_t e = launch_steps2d(ctx->stream, l.cls, planes[0].jobs.as<PlaneJob>(), planes[0].n, tab.as<float>(), tmaps.p,
                                            l.floats, runs, k, faces ? 1 : 0, stage_cells, ctx->status);
             if (e != cudaSuccess) return cuda_fail(ctx, e, "2-D steps launch");
             ctx->launches++;
@@ -1160,7 +1155,6 @@ uint64_t Diffusion::device_bytes() const
         for (const auto& l : rest[a]) b += l.tiles.bytes;
     for (const auto& pl : planes) b += pl.jobs.bytes;
     for (const auto& pl : zplanes) b += pl.jobs.bytes;
-    for (const auto& l : steps) b += l.jobs.bytes;
     return b;
 }
 
@@ -1360,7 +1354,7 @@ int Cells::create(pcg_ctx* c, uint32_t maxc, uint32_t rate_capacity, uint32_t n_
     PCG_CU(ctx, run_word.alloc((static_cast<size_t>(max_cells) + 1) * sizeof(uint64_t)));
     PCG_CU(ctx, inst_run.alloc(h_inst.size() * sizeof(uint32_t)));
     PCG_CU(ctx, cudaMemsetAsync(inst_run.p, 0, inst_run.bytes, ctx->stream));
-    PCG_CU(ctx, so_prepare());
+    PCG_CU(ctx, so_prepare(max_cells));
     max_tiles = so_max_tiles(max_cells, static_cast<uint32_t>(h_inst.size()));
     PCG_CU(ctx, tiles.alloc(static_cast<size_t>(max_tiles) * sizeof(SegTile)));
     PCG_CU(ctx, inst_tile.alloc(h_inst.size() * sizeof(uint32_t)));

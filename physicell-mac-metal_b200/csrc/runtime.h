@@ -175,10 +175,8 @@ struct PlaneList {
 
 // 2-D planes that take several sub-steps in one launch (k_steps_2d).
 struct StepList {
-    DevBuf jobs;
-    uint32_t n = 0;
     int cls = 0;               // steps2d_class
-    uint32_t floats = 0;       // largest plane_floats of the jobs
+    uint32_t floats = 0;       // plane_floats of the planes
 };
 
 struct SweepList {

@@ -666,12 +666,12 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
     }
 }
 
-cudaError_t so_prepare()
+// Only the largest tile is past the 48 KB that need no leave.
+cudaError_t so_prepare(uint32_t max_cells)
 {
-    cudaError_t e = allow_max_smem(reinterpret_cast<const void*>(k_so_cluster<1>));
-    if (e == cudaSuccess) e = allow_max_smem(reinterpret_cast<const void*>(k_so_cluster<2>));
-    if (e == cudaSuccess) e = allow_max_smem(reinterpret_cast<const void*>(k_so_cluster<kClusterMaxItems>));
-    return e;
+    static_assert(sizeof(ClusterSmem<2>) <= 48 * 1024, "launched without leave");
+    if (max_cells <= 2 * kClusterCtas * kClusterThreads) return cudaSuccess;
+    return allow_max_smem(reinterpret_cast<const void*>(k_so_cluster<kClusterMaxItems>));
 }
 
 // ------------------------------------------------------------------ host
