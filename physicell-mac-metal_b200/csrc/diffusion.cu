@@ -411,11 +411,21 @@ __host__ __device__ constexpr int long_stride() { return 32 * (K + 1) + 4; }   /
 template <int K>
 __device__ __forceinline__ int long_at(int i) { return i + i / K; }
 
+// One term of the scan's maps, G a + D.  The product G of many g below 1
+// underflows to 0, where a walk position by position would carry an infinite
+// a on undamped: such an a is multiplied by 'one' (1, or 0 where the rule has
+// no coupling and every g is 0) instead.
+__device__ __forceinline__ float long_term(float G, float a, float D, float one)
+{
+    return fmaf(fabsf(a) == INFINITY ? one : G, a, D);
+}
+
 // One direction of a line's segment: v[k] = h (forward) or d (backward) in,
 // the recurrence's values out; 'edge' enters at the segment's first
-// position in walking order.  Returns the value at the last one.
+// position in walking order; 'one' as in long_term.  Returns the value at
+// the last one.
 template <int K, bool BACK>
-__device__ __forceinline__ float long_scan(float (&v)[K], const float (&g)[K], float edge, int lane)
+__device__ __forceinline__ float long_scan(float (&v)[K], const float (&g)[K], float edge, float one, int lane)
 {
     float D = 0.f, G = 1.f;
 #pragma unroll
@@ -431,13 +441,13 @@ __device__ __forceinline__ float long_scan(float (&v)[K], const float (&g)[K], f
         const float Dp = BACK ? __shfl_down_sync(0xffffffffu, D, o) : __shfl_up_sync(0xffffffffu, D, o);
         const float Gp = BACK ? __shfl_down_sync(0xffffffffu, G, o) : __shfl_up_sync(0xffffffffu, G, o);
         if (pos >= o) {
-            D = fmaf(G, Dp, D);
+            D = long_term(G, Dp, D, one);
             G *= Gp;
         }
     }
     const float Dx = BACK ? __shfl_down_sync(0xffffffffu, D, 1) : __shfl_up_sync(0xffffffffu, D, 1);
     const float Gx = BACK ? __shfl_down_sync(0xffffffffu, G, 1) : __shfl_up_sync(0xffffffffu, G, 1);
-    float x = pos == 0 ? edge : fmaf(Gx, edge, Dx);
+    float x = pos == 0 ? edge : long_term(Gx, edge, Dx, one);
 #pragma unroll
     for (int q = 0; q < K; ++q) {
         const int k = BACK ? K - 1 - q : q;
@@ -521,11 +531,17 @@ __global__ void __launch_bounds__(32 * kLongLines) k_sweep_long(float* __restric
         __syncthreads();   // the stage may be loaded again
     };
 
+    const float one = n > 3 && __ldg(t + 1) > 0.f ? 1.f : 0.f;   // g of the first interior node: 0 without coupling
     if (n <= kSeg) {
         load(0);
         to_rhs(0);
-        long_scan<K, false>(v, g, 0.f, lane);
-        long_scan<K, true>(v, g, 0.f, lane);
+        long_scan<K, false>(v, g, 0.f, one, lane);
+        // the forward walk leaves 0 at the end node and past it, but NaN
+        // (0 times infinity) behind an infinite value
+#pragma unroll
+        for (int k = 0; k < K; ++k)
+            if (lane * K + k >= n - 1) v[k] = 0.f;
+        long_scan<K, true>(v, g, 0.f, one, lane);
         store(0, true);
         return;
     }
@@ -534,13 +550,13 @@ __global__ void __launch_bounds__(32 * kLongLines) k_sweep_long(float* __restric
     for (; s0 < n; s0 += kSeg) {
         load(s0);
         to_rhs(s0);
-        edge = long_scan<K, false>(v, g, edge, lane);
+        edge = long_scan<K, false>(v, g, edge, one, lane);
         store(s0, false);
     }
     edge = 0.f;
     for (s0 -= kSeg; s0 >= 0; s0 -= kSeg) {
         load(s0);
-        edge = long_scan<K, true>(v, g, edge, lane);
+        edge = long_scan<K, true>(v, g, edge, one, lane);
         store(s0, true);
     }
 }
