@@ -43,8 +43,8 @@ __global__ void k_sec_cell_consts(const float* __restrict__ soa, uint32_t stride
                                   const double* __restrict__ rates4, uint32_t n_rate, double dt,
                                   double* __restrict__ cc, uint32_t* __restrict__ flags)
 {
-    dependents_may_launch();
     if (!await_predecessors()) return;
+    dependents_may_launch();
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     const bool live = g < n;
     const unsigned live_lanes = __ballot_sync(0xFFFFFFFFu, live);   // blocks are whole warps
@@ -87,8 +87,8 @@ __global__ void k_sec_permute(const uint32_t* __restrict__ skeys, const uint32_t
                               uint32_t invalid_key, const uint32_t* __restrict__ flags,
                               const double* __restrict__ cc, uint32_t n_rate, double* __restrict__ cs)
 {
-    dependents_may_launch();
     if (!await_predecessors()) return;
+    dependents_may_launch();
     const uint32_t q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= n) return;
     if (skeys[q] >= invalid_key) return;
@@ -218,8 +218,7 @@ __global__ void __launch_bounds__(WIDE ? kWideBlock : 256, WIDE ? 5 : 6) k_secre
                           const CellInst* __restrict__ insts, const double* __restrict__ cs, uint64_t cap,
                           const uint32_t* __restrict__ flags, const uint8_t* __restrict__ mask)
 {
-    dependents_may_launch();
-    if (!await_predecessors()) return;
+    if (!await_predecessors()) return;   // its dependents, mostly planes, launch as its blocks end
     const uint32_t r = blockIdx.x * blockDim.x + threadIdx.x;
     if (r >= *n_runs) return;
     // a run's start and word (instance, the voxel's density element) were
@@ -344,8 +343,8 @@ __global__ void k_mech_bin(float* __restrict__ soa, uint32_t stride, uint32_t n,
                            uint32_t* __restrict__ slots, uint32_t* __restrict__ counts,
                            const uint8_t* __restrict__ mask)
 {
-    dependents_may_launch();
     if (!await_predecessors()) return;
+    dependents_may_launch();
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n) return;
     const uint32_t ii = cell_inst[g];
@@ -378,8 +377,8 @@ __global__ void k_mech_place(const float* __restrict__ soa, uint32_t stride, con
                              const uint32_t* __restrict__ slots, const uint32_t* __restrict__ start, uint32_t n,
                              uint2* __restrict__ placed)
 {
-    dependents_may_launch();
     if (!await_predecessors()) return;
+    dependents_may_launch();
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n) return;
     const float x = soa[static_cast<size_t>(F_POS_X) * stride + g];
@@ -431,8 +430,8 @@ __global__ void k_mech_order(const float* __restrict__ soa, uint32_t stride, con
                              const uint32_t* __restrict__ cell_inst, uint32_t* __restrict__ reach,
                              uint32_t* __restrict__ sorder, float4* __restrict__ spos, float4* __restrict__ sprm)
 {
-    dependents_may_launch();
     if (!await_predecessors()) return;
+    dependents_may_launch();
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     const bool live = g < n;
     uint32_t ii = 0, rb = 0;
@@ -468,8 +467,8 @@ __global__ void k_mech_order(const float* __restrict__ soa, uint32_t stride, con
 __global__ void k_mech_stable_order(const uint32_t* __restrict__ keys, const uint32_t* __restrict__ start,
                                     const uint2* __restrict__ placed, uint32_t n, uint32_t* __restrict__ sorder)
 {
-    dependents_may_launch();
     if (!await_predecessors()) return;
+    dependents_may_launch();
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n) return;
     const uint32_t key = keys[g];
@@ -581,8 +580,8 @@ __global__ void __launch_bounds__(256, WIDE ? 3 : 5) k_mech_forces(const float4*
                                                      uint32_t* __restrict__ diag_hash,
                                                      const uint8_t* __restrict__ mask)
 {
-    dependents_may_launch();
     if (!await_predecessors()) return;
+    dependents_may_launch();
     extern __shared__ uint32_t queue[];
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
@@ -752,8 +751,8 @@ __global__ void k_mech_integrate(float* __restrict__ soa, double* __restrict__ p
                                  const uint32_t* __restrict__ cell_inst, const CellInst* __restrict__ insts,
                                  float dt_override, const uint8_t* __restrict__ mask)
 {
-    dependents_may_launch();
     if (!await_predecessors()) return;
+    dependents_may_launch();
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= n) return;
     const uint32_t ii = cell_inst[g];

@@ -190,8 +190,8 @@ __global__ void __launch_bounds__(256, 1) k_sweep_tma(const SweepTile* __restric
                                                    int stage_floats, int nstages, int tab_area, int apply_faces,
                                                    const uint8_t* __restrict__ mask, unsigned* __restrict__ status)
 {
-    dependents_may_launch();
     if (!await_predecessors()) return;
+    dependents_may_launch();
     // stage: [tile data][tab_area floats of coefficient table]
     extern __shared__ __align__(128) unsigned char smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
@@ -293,7 +293,6 @@ __global__ void __launch_bounds__(256, 3)
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem);
     float* pl = reinterpret_cast<float*>(smem + 128);
-    dependents_may_launch();
     // the job, the tables and the tensor maps are written once, before any
     // step; the density and the mask may be the predecessor's
     const PlaneJob jb = jobs[blockIdx.x];
@@ -375,6 +374,7 @@ __global__ void __launch_bounds__(256, 3)
             if (last < nx) pl[j * P + last] = ry.T;
         }
     }
+    dependents_may_launch();   // late: waiting blocks take slots and issue from this one's solves
     fence_async_smem();
     __syncthreads();
     if (threadIdx.x == 0) {
@@ -463,8 +463,8 @@ __global__ void __launch_bounds__(32 * kLongLines) k_sweep_long(float* __restric
                                                                 const float* __restrict__ tab, int apply_faces,
                                                                 const uint8_t* __restrict__ mask)
 {
-    dependents_may_launch();
     if (!await_predecessors()) return;
+    dependents_may_launch();
     constexpr int kSeg = 32 * K, kStride = long_stride<K>();
     extern __shared__ float sh[];
     float* sg = sh + kLongLines * kStride;   // g of the segment's positions
@@ -565,8 +565,8 @@ __global__ void __launch_bounds__(32 * kLongLines) k_sweep_long(float* __restric
 
 __global__ void k_dirichlet(float* __restrict__ dens, const FaceJob* __restrict__ jobs)
 {
-    dependents_may_launch();
     if (!await_predecessors()) return;
+    dependents_may_launch();
     const FaceJob jb = jobs[blockIdx.x];
     float* base = dens + jb.base;
     const uint32_t nx = jb.nx, ny = jb.ny, nz = jb.nz;

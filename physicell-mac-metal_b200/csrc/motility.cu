@@ -105,8 +105,8 @@ __device__ __forceinline__ double norm3(double x, double y, double z)
 __global__ void k_motility(float* __restrict__ soa, uint32_t stride, MotState m, DensView dv, bool have_density,
                            double dt, uint64_t seed, uint64_t step, int layout)
 {
-    dependents_may_launch();
     if (!await_predecessors()) return;
+    dependents_may_launch();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m.n) return;
     if (__float_as_uint(soa[static_cast<size_t>(F_IS_ALIVE) * stride + i]) == 0u) return;

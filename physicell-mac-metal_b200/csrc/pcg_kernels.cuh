@@ -156,17 +156,27 @@ enum : uint8_t { STEP_DIFFUSE = 1u, STEP_MECH = 2u };
 // A step is a chain of short kernels, and between two of them the GPU idles
 // for 1-2 us (drain, launch, block start-up).  Every kernel of the chains is
 // launched with programmatic stream serialisation: once all blocks of its
-// predecessor have started (dependents_may_launch at their first statement)
-// its blocks take free slots, run what does not depend on the predecessor,
-// and wait (await_predecessors) until it has completed and its writes are
-// visible.  Every block of every kernel waits before it returns, so a
-// kernel's completion implies that of all before it.  In front of anything
-// else (a copy, an event wait) the launch orders itself as usual.  One
-// mechanics period of the 50 x 50 simulation 133 -> 82.5 us, a mechanics
-// update of 100k cells 67.8 -> 52.9 us.  Captured launches (a batch's
-// graphs) keep full edges: with parallel branches the waiting blocks take
-// slots from the branches still running (64 3-D instances 3.69 -> 3.90 ms
-// a period with programmatic edges, 256 2-D ones 1.53 -> 1.69).
+// predecessor have let it (dependents_may_launch), its blocks take free
+// slots, run what does not depend on the predecessor, and wait
+// (await_predecessors) until it has completed and its writes are visible.
+// Every block of every kernel waits before it returns, so a kernel's
+// completion implies that of all before it.  In front of anything else (a
+// copy, an event wait) the launch orders itself as usual.  One mechanics
+// period of the 50 x 50 simulation 133 -> 82.5 us, a mechanics update of
+// 100k cells 67.8 -> 50.5 us.
+//   A kernel lets its dependents launch only after its own wait, so at most
+// one kernel of the chain waits on the SMs.  When each let the next one
+// launch at its first statement, kernels several steps ahead filled the SMs
+// with waiting blocks and the running ones started late: a diffusion step of
+// 100^3 voxels 22.9 us against 11.0, of 80^3 on three substrates 20.9 against
+// 13.0 (14.4 both with plain launches), a sort of 200003 pairs 30.5 against
+// 22.9.  The plane kernel lets them launch once its lines are solved and the
+// secretion as its blocks end: what waits beside them is mostly a plane pass,
+// whose blocks are large (a period of 61 x 47 x 53 voxels 187 -> 173 us).
+//   Captured launches (a batch's graphs) keep full edges: with parallel
+// branches the waiting blocks take slots from the branches still running (64
+// 3-D instances 3.69 -> 3.90 ms a period with programmatic edges, 256 2-D
+// ones 1.53 -> 1.69).
 __device__ __forceinline__ void dependents_may_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // False never (a grid has at least one block in z); the branch on it keeps

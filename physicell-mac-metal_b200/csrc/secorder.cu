@@ -65,8 +65,8 @@ __global__ void __launch_bounds__(kThreads) k_so_hist(const SegTile* __restrict_
                                                       const uint8_t* __restrict__ active, uint32_t* __restrict__ keys,
                                                       int shift, uint32_t R, uint32_t* __restrict__ hist)
 {
-    dependents_may_launch();
     if (!await_predecessors()) return;
+    dependents_may_launch();
     __shared__ uint32_t cnt[kMaxBins];
     const SegTile tl = tiles[blockIdx.x];
     for (uint32_t d = threadIdx.x; d <= R; d += kThreads) cnt[d] = 0;
@@ -108,8 +108,8 @@ __global__ void __launch_bounds__(kOffThreads, 1) k_so_offsets(const SegTile* __
                                                             const CellInst* __restrict__ insts, uint32_t R,
                                                             uint32_t* __restrict__ hist)
 {
-    dependents_may_launch();
     if (!await_predecessors()) return;
+    dependents_may_launch();
     __shared__ uint32_t wsum[kOffThreads / 32];
     __shared__ uint32_t rows[kOffSmem / 4];
     const SegTile t0 = tiles[inst_tile[blockIdx.x]];
@@ -199,8 +199,8 @@ __global__ void __launch_bounds__(kThreads) k_so_scatter(const SegTile* __restri
                                                          const double* __restrict__ cc, double* __restrict__ cs,
                                                          uint32_t cap, const uint32_t* __restrict__ flags)
 {
-    dependents_may_launch();
     if (!await_predecessors()) return;
+    dependents_may_launch();
     __shared__ uint32_t wcnt[kWarps][kMaxBins];
     __shared__ uint32_t cnt[kMaxBins];
     __shared__ uint32_t tbase[kMaxBins];
@@ -341,8 +341,8 @@ __device__ __forceinline__ bool so_head(const uint32_t* __restrict__ skeys, uint
 __global__ void __launch_bounds__(kThreads) k_so_run_count(const uint32_t* __restrict__ skeys, uint32_t n,
                                                            uint32_t* __restrict__ tile_cnt)
 {
-    dependents_may_launch();
     if (!await_predecessors()) return;
+    dependents_may_launch();
     __shared__ uint32_t ws[kWarps];
     uint32_t c = 0, key;
 #pragma unroll
@@ -368,8 +368,8 @@ __global__ void __launch_bounds__(kThreads) k_so_run_write(const uint32_t* __res
                                                            uint64_t* __restrict__ run_word, uint32_t* __restrict__ n_runs,
                                                            uint32_t* __restrict__ inst_run)
 {
-    dependents_may_launch();
     if (!await_predecessors()) return;
+    dependents_may_launch();
     __shared__ uint32_t wc[kItems * kWarps];   // heads per (row k, warp), then their exclusive scan
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint32_t lt_mask = (1u << lane) - 1u;
@@ -501,8 +501,8 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
     constexpr uint32_t kOwn = ClusterSmem<I>::kOwn;
     extern __shared__ __align__(16) unsigned char so_smem[];
     ClusterSmem<I>& m = *reinterpret_cast<ClusterSmem<I>*>(so_smem);
-    dependents_may_launch();
     if (!await_predecessors()) return;
+    dependents_may_launch();
     const uint32_t rank = blockIdx.x;   // one cluster: the block's rank in it
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t lt_mask = (1u << lane) - 1u;

@@ -36,8 +36,8 @@ constexpr uint32_t kMask = kRadix - 1;
 __global__ void __launch_bounds__(kThreads) k_radix_hist(const uint32_t* __restrict__ keys, uint32_t n, int shift,
                                                          uint32_t* __restrict__ hist)
 {
-    dependents_may_launch();
     if (!await_predecessors()) return;
+    dependents_may_launch();
     __shared__ uint32_t h[kRadix];
     for (int i = threadIdx.x; i < kRadix; i += kThreads) h[i] = 0;
     __syncthreads();
@@ -61,8 +61,8 @@ __global__ void __launch_bounds__(kThreads) k_radix_scatter(const uint32_t* __re
                                                             uint32_t n, int shift,
                                                             const uint32_t* __restrict__ hist, uint32_t ntiles)
 {
-    dependents_may_launch();
     if (!await_predecessors()) return;
+    dependents_may_launch();
     __shared__ uint32_t wcnt[kWarps][kRadix];
     __shared__ uint32_t gbase[kRadix];
     __shared__ uint32_t tbase[kRadix];      // first place of each digit in the tile
@@ -212,8 +212,8 @@ constexpr uint64_t kOneBlock = 4ull * kOneItems * kOneThreads;   // 32768
 __global__ void __launch_bounds__(kOneThreads) k_scan_one(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
                                                           uint32_t n)
 {
-    dependents_may_launch();
     if (!await_predecessors()) return;
+    dependents_may_launch();
     __shared__ uint32_t wtot[kOneItems * 32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool aligned = ((reinterpret_cast<uintptr_t>(in) | reinterpret_cast<uintptr_t>(out)) & 15u) == 0;
@@ -282,8 +282,8 @@ __global__ void __launch_bounds__(kOneThreads) k_scan_one(const uint32_t* __rest
 __global__ void __launch_bounds__(kThreads) k_tile_sums(const uint32_t* __restrict__ in, uint64_t n,
                                                         uint32_t* __restrict__ sums)
 {
-    dependents_may_launch();
     if (!await_predecessors()) return;
+    dependents_may_launch();
     __shared__ uint32_t wsum[kWarps];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const uint64_t base = static_cast<uint64_t>(blockIdx.x) * kTile + static_cast<uint64_t>(threadIdx.x) * kItems;
@@ -344,8 +344,8 @@ __device__ __forceinline__ uint32_t block_exclusive(uint32_t x, uint32_t* wsum, 
 __global__ void __launch_bounds__(kThreads) k_scan_tiles(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
                                                          uint64_t n, const uint32_t* __restrict__ offs)
 {
-    dependents_may_launch();
     if (!await_predecessors()) return;
+    dependents_may_launch();
     static_assert(kTile == 2 * 4 * kThreads, "two halves of four values per thread");
     __shared__ uint32_t wsum[kWarps + 1];
     const uint64_t tile = static_cast<uint64_t>(blockIdx.x) * kTile;

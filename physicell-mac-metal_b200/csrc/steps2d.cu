@@ -245,7 +245,6 @@ __global__ void __launch_bounds__(kSteps2dThreads) k_steps_2d(const PlaneJob* __
     extern __shared__ __align__(128) unsigned char smem[];
     uint64_t* bar = reinterpret_cast<uint64_t*>(smem);
     float* pl = reinterpret_cast<float*>(smem + 128);
-    dependents_may_launch();
     const PlaneJob jb = jobs[blockIdx.x];
     const uint32_t ii = jb.inst & kPlaneInstMask;
     const uint32_t nx = jb.nx, ny = jb.ny, P = plane_pitch(nx, false);
@@ -258,6 +257,7 @@ __global__ void __launch_bounds__(kSteps2dThreads) k_steps_2d(const PlaneJob* __
         asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory");
     }
     if (!await_predecessors()) return;
+    dependents_may_launch();
     __syncthreads();
     if (threadIdx.x == 0) {
         const uint32_t tbx = tab_floats(nx) * 4u, tby = tab_floats(ny) * 4u;
