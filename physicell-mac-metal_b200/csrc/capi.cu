@@ -19,10 +19,18 @@ thread_local std::string g_create_err;
 int bad(pcg_ctx* ctx, const char* msg) { return fail(ctx, PCG_ERR_INVALID, msg); }
 
 // Most cells of a single 2-D simulation whose secretion runs inside its
-// plane's CTAs (pcg_me_step): they share S SMs there, the whole GPU in a
-// launch of their own.  10 sub-steps of 50 x 50: 25.5 us fused against 65.5
-// at 500 cells, 73.1 against 71.9 at 5000.
-constexpr uint32_t kFusedStepCells = 4096;
+// plane's CTAs in a call of n_steps (pcg_me_step).  There they share S SMs,
+// where a launch of their own has the whole GPU, and their runs and terms are
+// staged first, so each sub-step pays for a number of cells.  Fused time over
+// separate, sides 20 to 230, one to four substrates, one to 16 cells a voxel
+// and crowded, geometric mean (range): one sub-step, 100 cells 0.87 (0.58 -
+// 0.97), 250 1.04 (0.91 - 1.36), 4096 1.80; two, 1000 cells 0.89 (0.64 -
+// 1.16), 2000 1.04 (0.60 - 1.38), 4096 1.18 (up to 2.1); three, 2000 0.90,
+// 4096 1.06; five, 3000 0.98, 4096 0.95 (0.37 - 1.42); ten, 4096 0.87.
+uint32_t fused_step_cells(int n_steps)
+{
+    return n_steps <= 1 ? 128u : n_steps >= 5 ? 4096u : 1024u * static_cast<uint32_t>(n_steps - 1);
+}
 
 bool same_bytes(const void* a, const void* b, size_t n) { return std::memcmp(a, b, n) == 0; }
 
@@ -316,7 +324,7 @@ pcg_status pcg_me_step(pcg_me* me, pcg_cells* cells, int n_steps)
         PCG_TRY(bind_me(cells, me));
     }
     const double dt = me->d.inst[0].g.dt;
-    if (me->d.takes_steps(n_steps) && (!sec || (cells->c.n <= kFusedStepCells && me->d.steps_fit(cells->c.n)))) {
+    if (me->d.takes_steps(n_steps) && (!sec || (cells->c.n <= fused_step_cells(n_steps) && me->d.steps_fit(cells->c.n)))) {
         // a 2-D plane: all sub-steps in one launch
         if (sec) PCG_TRY(cells->c.prepare_secretion(dt, me->d.total_vox));
         return me->d.steps_2d(n_steps, true, sec ? cells->c.run_args() : RunArgs{}, sec ? cells->c.n : 0);
