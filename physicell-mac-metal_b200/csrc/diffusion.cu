@@ -411,43 +411,55 @@ __host__ __device__ constexpr int long_stride() { return 32 * (K + 1) + 4; }   /
 template <int K>
 __device__ __forceinline__ int long_at(int i) { return i + i / K; }
 
-// One term of the scan's maps, G a + D.  The product G of many g below 1
-// underflows to 0, where a walk position by position would carry an infinite
-// a on undamped: such an a is multiplied by 'one' (1, or 0 where the rule has
-// no coupling and every g is 0) instead.
-__device__ __forceinline__ float long_term(float G, float a, float D, float one)
+// Inclusive scan of a segment's affine maps (D, G) over the lanes, in walking
+// order; 'term' gives one map's G a + D.
+template <bool BACK, class TERM>
+__device__ __forceinline__ void scan_maps(float& D, float& G, int pos, TERM term)
 {
-    return fmaf(fabsf(a) == INFINITY ? one : G, a, D);
-}
-
-// One direction of a line's segment: v[k] = h (forward) or d (backward) in,
-// the recurrence's values out; 'edge' enters at the segment's first
-// position in walking order; 'one' as in long_term.  Returns the value at
-// the last one.
-template <int K, bool BACK>
-__device__ __forceinline__ float long_scan(float (&v)[K], const float (&g)[K], float edge, float one, int lane)
-{
-    float D = 0.f, G = 1.f;
-#pragma unroll
-    for (int q = 0; q < K; ++q) {
-        const int k = BACK ? K - 1 - q : q;
-        D = fmaf(g[k], D, v[k]);
-        G *= g[k];
-    }
-    // inclusive scan of the affine maps in walking order
-    const int pos = BACK ? 31 - lane : lane;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const float Dp = BACK ? __shfl_down_sync(0xffffffffu, D, o) : __shfl_up_sync(0xffffffffu, D, o);
         const float Gp = BACK ? __shfl_down_sync(0xffffffffu, G, o) : __shfl_up_sync(0xffffffffu, G, o);
         if (pos >= o) {
-            D = long_term(G, Dp, D, one);
+            D = term(G, Dp, D);
             G *= Gp;
         }
     }
+}
+
+// One direction of a line's segment: v[k] = h (forward) or d (backward) in,
+// the recurrence's values out; 'edge' enters at the segment's first
+// position in walking order.  Returns the value at the last one.
+//   The product G of many g below 1 underflows to 0, and 0 times an infinite
+// value would be NaN where a walk position by position carries it on undamped.
+// So where a value is not finite ('wild' is set) the scan is run again with
+// an infinite a multiplied by 'one' instead: 1, or 0 where the rule has no
+// coupling and every g is 0.
+template <int K, bool BACK>
+__device__ __forceinline__ float long_scan(float (&v)[K], const float (&g)[K], float edge, float one, bool& wild, int lane)
+{
+    float D, G;
+    auto run = [&]() {   // the lane's positions from zero
+        D = 0.f;
+        G = 1.f;
+#pragma unroll
+        for (int q = 0; q < K; ++q) {
+            const int k = BACK ? K - 1 - q : q;
+            D = fmaf(g[k], D, v[k]);
+            G *= g[k];
+        }
+    };
+    const int pos = BACK ? 31 - lane : lane;
+    run();
+    scan_maps<BACK>(D, G, pos, [](float m, float a, float d) { return fmaf(m, a, d); });
+    wild = __any_sync(0xffffffffu, !(fabsf(D) < INFINITY) || !(fabsf(edge) < INFINITY));
+    if (wild) {
+        run();
+        scan_maps<BACK>(D, G, pos, [one](float m, float a, float d) { return fmaf(fabsf(a) == INFINITY ? one : m, a, d); });
+    }
     const float Dx = BACK ? __shfl_down_sync(0xffffffffu, D, 1) : __shfl_up_sync(0xffffffffu, D, 1);
     const float Gx = BACK ? __shfl_down_sync(0xffffffffu, G, 1) : __shfl_up_sync(0xffffffffu, G, 1);
-    float x = pos == 0 ? edge : long_term(Gx, edge, Dx, one);
+    float x = pos == 0 ? edge : fmaf(wild && fabsf(edge) == INFINITY ? one : Gx, edge, Dx);
 #pragma unroll
     for (int q = 0; q < K; ++q) {
         const int k = BACK ? K - 1 - q : q;
@@ -535,28 +547,32 @@ __global__ void __launch_bounds__(32 * kLongLines) k_sweep_long(float* __restric
     if (n <= kSeg) {
         load(0);
         to_rhs(0);
-        long_scan<K, false>(v, g, 0.f, one, lane);
+        bool wild;
+        long_scan<K, false>(v, g, 0.f, one, wild, lane);
         // the forward walk leaves 0 at the end node and past it, but NaN
         // (0 times infinity) behind an infinite value
+        if (wild) {
 #pragma unroll
-        for (int k = 0; k < K; ++k)
-            if (lane * K + k >= n - 1) v[k] = 0.f;
-        long_scan<K, true>(v, g, 0.f, one, lane);
+            for (int k = 0; k < K; ++k)
+                if (lane * K + k >= n - 1) v[k] = 0.f;
+        }
+        long_scan<K, true>(v, g, 0.f, one, wild, lane);
         store(0, true);
         return;
     }
     float edge = 0.f;
+    bool wild;
     int s0 = 0;
     for (; s0 < n; s0 += kSeg) {
         load(s0);
         to_rhs(s0);
-        edge = long_scan<K, false>(v, g, edge, one, lane);
+        edge = long_scan<K, false>(v, g, edge, one, wild, lane);
         store(s0, false);
     }
     edge = 0.f;
     for (s0 -= kSeg; s0 >= 0; s0 -= kSeg) {
         load(s0);
-        edge = long_scan<K, true>(v, g, edge, one, lane);
+        edge = long_scan<K, true>(v, g, edge, one, wild, lane);
         store(s0, true);
     }
 }
