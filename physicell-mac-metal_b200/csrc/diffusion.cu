@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(256, 3)
 
 // Lines too long for a tensor box (and any line without a tensor map): one
 // warp per line, kLongLines lines per CTA (8 adjacent columns: one 32-byte
-// sector per row).  Both recurrences are affine, d_i = g_i d_{i-1} + h_i and
+// sector per row), 'parts' CTAs per tile of up to 32 lines.  Both recurrences are affine, d_i = g_i d_{i-1} + h_i and
 // x_i = g_i x_{i+1} + d_i, so lane l takes K consecutive positions, runs
 // them from zero, the 32 (product of g, end value) pairs are scanned with
 // shuffles, and the lane runs its positions again from the value the scan
@@ -471,7 +471,7 @@ __device__ __forceinline__ float long_scan(float (&v)[K], const float (&g)[K], f
 
 template <int K>
 __global__ void __launch_bounds__(32 * kLongLines) k_sweep_long(float* __restrict__ dens,
-                                                                const SweepTile* __restrict__ tiles,
+                                                                const SweepTile* __restrict__ tiles, uint32_t parts,
                                                                 const float* __restrict__ tab, int apply_faces,
                                                                 const uint8_t* __restrict__ mask)
 {
@@ -481,9 +481,10 @@ __global__ void __launch_bounds__(32 * kLongLines) k_sweep_long(float* __restric
     extern __shared__ float sh[];
     float* sg = sh + kLongLines * kStride;   // g of the segment's positions
     float* si = sg + kStride;                // 1 / den
-    const SweepTile tile = tiles[blockIdx.x];
+    const SweepTile tile = tiles[blockIdx.x / parts];
+    const uint32_t l0 = blockIdx.x % parts * kLongLines;   // the CTA's first line of the tile
     const LineRule r = rule_of(tile);
-    if (!tile_on(r, mask)) return;   // the whole CTA leaves together
+    if (l0 >= tile.count || !tile_on(r, mask)) return;   // the whole CTA leaves together
     const int n = static_cast<int>(r.n), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool rows = (tile.face & TILE_ROWS) != 0;
     const float* t = tab + r.tab + seq_table_offset(r.n);
@@ -491,11 +492,11 @@ __global__ void __launch_bounds__(32 * kLongLines) k_sweep_long(float* __restric
     // warp; columns, 8 adjacent lines per row of threads
     const int line = rows ? warp : static_cast<int>(threadIdx.x & 7u);
     const int p0 = rows ? lane : static_cast<int>(threadIdx.x >> 3), dp = 32;
-    const bool mine = line < static_cast<int>(tile.count);
+    const bool mine = l0 + line < tile.count;
     const size_t ls = rows ? tile.rs : 1, ps = rows ? 1 : tile.rs;
-    float* gl = dens + tile.base + static_cast<size_t>(line) * ls;
+    float* gl = dens + tile.base + static_cast<size_t>(l0 + line) * ls;
     float* sl = sh + line * kStride;
-    const bool face = !rows && apply_faces && (tile.face & TILE_FACE) && mine && on_face(tile, line);
+    const bool face = !rows && apply_faces && (tile.face & TILE_FACE) && mine && on_face(tile, static_cast<int>(l0) + line);
     const float* sv = sh + warp * kStride + lane * (K + 1);
     float* sw = sh + warp * kStride + lane * (K + 1);
     float v[K], g[K];
@@ -827,25 +828,26 @@ cudaError_t launch_sweep_planes(cudaStream_t st, bool z, int threads, const Plan
 }
 
 template <int K>
-static cudaError_t long_variant(cudaStream_t st, float* dens, const SweepTile* tiles, uint32_t ntiles, const float* tab,
-                                int apply_faces, const uint8_t* mask)
+static cudaError_t long_variant(cudaStream_t st, float* dens, const SweepTile* tiles, uint32_t ntiles, uint32_t parts,
+                                const float* tab, int apply_faces, const uint8_t* mask)
 {
     const size_t smem = static_cast<size_t>(kLongLines + 2) * long_stride<K>() * sizeof(float);   // at most 43 KB
-    launch_chained(st, k_sweep_long<K>, ntiles, 32 * kLongLines, smem, dens, tiles, tab, apply_faces, mask);
+    launch_chained(st, k_sweep_long<K>, ntiles * parts, 32 * kLongLines, smem, dens, tiles, parts, tab, apply_faces, mask);
     return cudaGetLastError();
 }
 
-cudaError_t launch_sweep_long(cudaStream_t st, float* dens, const SweepTile* tiles, uint32_t ntiles, const float* tab,
-                              int nmax, int apply_faces, const uint8_t* mask)
+cudaError_t launch_sweep_long(cudaStream_t st, float* dens, const SweepTile* tiles, uint32_t ntiles, uint32_t lines,
+                              const float* tab, int nmax, int apply_faces, const uint8_t* mask)
 {
     if (ntiles == 0) return cudaSuccess;
+    const uint32_t parts = (lines + kLongLines - 1) / kLongLines;
     // positions per lane: the fewest that hold the longest line in one
     // segment (a lane's steps, registers and shared memory grow with them),
     // at most 32; longer lines take several segments
-    if (nmax <= 32 * 12) return long_variant<12>(st, dens, tiles, ntiles, tab, apply_faces, mask);
-    if (nmax <= 32 * 16) return long_variant<16>(st, dens, tiles, ntiles, tab, apply_faces, mask);
-    if (nmax <= 32 * 24) return long_variant<24>(st, dens, tiles, ntiles, tab, apply_faces, mask);
-    return long_variant<32>(st, dens, tiles, ntiles, tab, apply_faces, mask);
+    if (nmax <= 32 * 12) return long_variant<12>(st, dens, tiles, ntiles, parts, tab, apply_faces, mask);
+    if (nmax <= 32 * 16) return long_variant<16>(st, dens, tiles, ntiles, parts, tab, apply_faces, mask);
+    if (nmax <= 32 * 24) return long_variant<24>(st, dens, tiles, ntiles, parts, tab, apply_faces, mask);
+    return long_variant<32>(st, dens, tiles, ntiles, parts, tab, apply_faces, mask);
 }
 
 cudaError_t launch_dirichlet(cudaStream_t st, float* dens, const FaceJob* jobs, uint32_t njobs)

@@ -76,9 +76,9 @@ __host__ __device__ constexpr uint32_t seq_table_floats(uint32_t n) { return ((n
 // (the row pitch) apart.  Column tiles (y and z sweeps): 'nslab' adjacent
 // slabs (outer coordinates outer .. outer + nslab - 1) of 'count' (<= width)
 // adjacent columns from x = i0, width * nslab <= 32; lane = slab * width +
-// column.  Tiles without TILE_TENSOR (k_sweep_long) hold up to kLongLines
-// lines: rows as above, columns of one slab (width kLongLines) starting at
-// 'base' with element stride 'rs'.
+// column.  Tiles of lines without a tensor map (k_sweep_long): rows as
+// above, columns of one slab (width 32) starting at 'base' with element
+// stride 'rs'.
 struct SweepTile {
     uint64_t base;
     uint32_t count;
@@ -344,10 +344,10 @@ bool encode_column_map(void* map128, float* block, uint32_t nx, uint32_t ny, uin
 // Encode the 2-D tensor map of one substrate block seen as rows x nx (rows
 // px floats apart) with a box of row_smem_pitch(nx) x 32 (x tiles).
 bool encode_row_map(void* map128, float* block, uint32_t nx, uint64_t rows, uint32_t px);
-// Any line length, one warp per line, one CTA per tile of up to kLongLines
-// lines; nmax = the longest line of the tiles.
-cudaError_t launch_sweep_long(cudaStream_t st, float* dens, const SweepTile* tiles, uint32_t ntiles, const float* tab,
-                              int nmax, int apply_faces, const uint8_t* mask);
+// Any line length, one warp per line, kLongLines lines per CTA; lines = the
+// most lines of a tile (at most 32), nmax = the longest line of the tiles.
+cudaError_t launch_sweep_long(cudaStream_t st, float* dens, const SweepTile* tiles, uint32_t ntiles, uint32_t lines,
+                              const float* tab, int nmax, int apply_faces, const uint8_t* mask);
 
 // applyDirichletBC over instances [0, n_inst): faces of Dirichlet substrates.
 struct FaceJob { uint64_t base; uint32_t nx, ny, nz, px; float T; uint32_t _pad; };

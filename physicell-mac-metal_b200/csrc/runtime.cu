@@ -783,12 +783,11 @@ int Diffusion::build_axis(int axis, const std::vector<uint8_t>* skip, std::vecto
             nmax = std::max<int>(nmax, static_cast<int>(n));
             if (axis == 0) {
                 const uint64_t lines = d.rows();
-                const uint64_t per = fast ? 32 : kLongLines;
-                for (uint64_t l0 = 0; l0 < lines; l0 += per) {
+                for (uint64_t l0 = 0; l0 < lines; l0 += 32) {
                     SweepTile t{};
                     t.base = sbase + l0 * d.px;
                     fill_rule(t, h_rules_[rule]);
-                    t.count = static_cast<uint32_t>(std::min<uint64_t>(per, lines - l0));
+                    t.count = static_cast<uint32_t>(std::min<uint64_t>(32, lines - l0));
                     t.rs = d.px;
                     t.nx = g.nx;
                     t.outer = static_cast<uint32_t>(l0);
@@ -807,11 +806,10 @@ int Diffusion::build_axis(int axis, const std::vector<uint8_t>* skip, std::vecto
                 const uint32_t outer = axis == 1 ? g.nz : g.ny;
                 const uint64_t ostride = axis == 1 ? static_cast<uint64_t>(d.px) * g.ny : d.px;
                 const uint32_t rs = axis == 1 ? d.px : d.px * g.ny;
-                const uint32_t per = fast ? 32u : kLongLines;
-                for (uint32_t i0 = 0; i0 < g.nx; i0 += per) {
-                    const uint32_t cnt = std::min<uint32_t>(per, g.nx - i0);
+                for (uint32_t i0 = 0; i0 < g.nx; i0 += 32) {
+                    const uint32_t cnt = std::min<uint32_t>(32, g.nx - i0);
                     const int w = !fast || cnt > 16 ? 0 : cnt > 8 ? 1 : 2;
-                    const uint32_t width = fast ? 32u >> w : kLongLines;
+                    const uint32_t width = 32u >> w;
                     const uint32_t group = fast ? 32u / width : 1u;
                     for (uint32_t o = 0; o < outer; o += group) {
                         SweepTile t{};
@@ -852,6 +850,7 @@ int Diffusion::build_axis(int axis, const std::vector<uint8_t>* skip, std::vecto
     ls[1].n = static_cast<uint32_t>(long_t.size());
     ls[1].lines = long_lines;
     ls[1].units = long_units;
+    for (const SweepTile& t : long_t) ls[1].count = std::max(ls[1].count, t.count);
     for (int q = 0; q < 2; ++q) {
         const auto& v = q == 0 ? fast_t : long_t;
         PCG_CU(ctx, ls[q].tiles.alloc(std::max<size_t>(v.size(), 1) * sizeof(SweepTile)));
@@ -937,7 +936,7 @@ int Diffusion::launch_list(const SweepList& l, bool fuse, const uint8_t* mask)
     const SweepTile* t = l.tiles.as<SweepTile>();
     const float* tb = tab.as<float>();
     cudaError_t e;
-    if (l.kind == 2) e = launch_sweep_long(ctx->stream, d, t, l.n, tb, l.nmax, fuse ? 1 : 0, mask);
+    if (l.kind == 2) e = launch_sweep_long(ctx->stream, d, t, l.n, l.count, tb, l.nmax, fuse ? 1 : 0, mask);
     else
         e = launch_sweep_tma(ctx->stream, l.kind == 0, t, l.n, tb, tmaps.p, fuse ? 1 : 0, mask, ctx->status, l.tc);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "sweep launch");
@@ -1171,9 +1170,9 @@ std::string Diffusion::describe() const
             o << ax[a] << ":";
             if (l.kind != 2)
                 o << (l.kind == 0 ? "x-tma(" : "cols-tma(") << "warps=" << l.tc.warps << ",stages=" << l.tc.stages
-                  << ",grid=" << l.tc.grid;
+                  << ",grid=" << l.tc.grid << ",";
             else o << "warp-lines(";
-            o << ",tiles=" << l.n << ",nmax=" << l.nmax << ") ";
+            o << "tiles=" << l.n << ",nmax=" << l.nmax << ") ";
         }
     return o.str();
 }

@@ -183,6 +183,7 @@ struct SweepList {
     int kind = 0;              // 0 row tiles (TMA), 1 column tiles (TMA), 2 any length (one warp per line)
     int nmax = 0;
     uint32_t n = 0;
+    uint32_t count = 0;        // most lines of a tile (kind 2)
     DevBuf tiles;
     TmaCfg tc{4, 3, 0, 1};
     uint64_t lines = 0;        // lines covered (for tuning keys)
