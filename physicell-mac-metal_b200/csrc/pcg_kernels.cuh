@@ -280,12 +280,11 @@ __host__ __device__ constexpr uint32_t plane_floats(uint32_t nx, uint32_t ny, bo
 // cls: the most chunks of a half line that stay in registers (8: planes of
 // sides up to 64, 16: up to 128, two lanes per line; 0: any, one thread per
 // line in shared memory).  Secretion reads the run list of the secretion
-// order; run_word null: none.
+// order of the one instance; run_word null: none.
 struct RunArgs {
     const uint32_t* run_start = nullptr;
     const uint64_t* run_word = nullptr;
     const uint32_t* n_runs = nullptr;
-    const uint32_t* inst_run = nullptr;
     const CellInst* insts = nullptr;
     const double* cs = nullptr;
     uint64_t cap = 0;
@@ -458,8 +457,7 @@ size_t so_run_scratch_bytes(uint32_t max_cells);
 cudaError_t so_prepare(uint32_t max_cells);   // before the first order of a store of max_cells
 // Keys, the sort and the run list in one call.  Outputs: skeys (global
 // voxel key vox_base + index, or invalid_key) and sorder (cell) per sorted
-// position; *n_runs; run_start (n + 1) and run_word per run; inst_run per
-// instance with secreting cells, its first run.  keys, ktmp
+// position; *n_runs; run_start (n + 1) and run_word per run.  keys, ktmp
 // and vtmp are n-entry work arrays;
 // scratch: so_scratch_bytes, run_scratch: so_run_scratch_bytes; inst_tile:
 // the n_inst_tiled entries of so_tiles.  With cc non-null the last pass
@@ -470,7 +468,7 @@ cudaError_t launch_sec_order(cudaStream_t st, const SegTile* tiles, uint32_t nti
                              int digit_bits, const float* soa, uint32_t stride, const CellInst* insts,
                              const uint8_t* active, const uint32_t* cell_inst, uint32_t invalid_key, uint32_t* keys,
                              uint32_t* ktmp, uint32_t* vtmp, uint32_t* skeys, uint32_t* sorder, void* scratch,
-                             uint32_t* n_runs, uint32_t* run_start, uint64_t* run_word, uint32_t* inst_run, void* run_scratch,
+                             uint32_t* n_runs, uint32_t* run_start, uint64_t* run_word, void* run_scratch,
                              const double* cc, double* cs, uint32_t cap, const uint32_t* flags);
 
 // Radix sort of (key, value) pairs, stable, 'bits' significant key bits.

@@ -721,17 +721,15 @@ int Diffusion::build_planes()
     return prepare_forks();
 }
 
-// The step list of a single 2-D simulation: its planes are one size, so they
+// The fused steps of a single 2-D simulation: its planes are one size, so they
 // are one plane list, whose jobs the steps share.
 int Diffusion::build_steps()
 {
-    steps.clear();
-    if (inst.size() != 1 || inst[0].ndim() != 2 || planes.size() != 1) return PCG_OK;
-    steps.emplace_back();
-    StepList& l = steps.back();
-    l.cls = steps2d_class(std::max(inst[0].g.nx, inst[0].g.ny));
-    l.floats = plane_floats(inst[0].g.nx, inst[0].g.ny);
-    PCG_CU(ctx, steps2d_prepare(l.cls));
+    steps.on = inst.size() == 1 && inst[0].ndim() == 2 && planes.size() == 1;
+    if (!steps.on) return PCG_OK;
+    steps.cls = steps2d_class(std::max(inst[0].g.nx, inst[0].g.ny));
+    steps.floats = plane_floats(inst[0].g.nx, inst[0].g.ny);
+    PCG_CU(ctx, steps2d_prepare(steps.cls));
     return PCG_OK;
 }
 
@@ -740,7 +738,7 @@ int Diffusion::build_steps()
 // more than the plane pass in calls of 1).
 bool Diffusion::takes_steps(int n) const
 {
-    return n > 0 && !steps.empty() && (n > 1 || (steps.size() == 1 && steps[0].cls == 8));
+    return n > 0 && steps.on && (n > 1 || steps.cls == 8);
 }
 
 // Copy a line rule into a tile descriptor.
@@ -992,23 +990,16 @@ int Diffusion::launch_planes(const std::vector<PlaneList>& pls, bool fuse, const
 // A launch runs at most this many sub-steps, so that a kernel stays short.
 static constexpr int kMaxFusedSteps = 256;
 
-bool Diffusion::steps_fit(uint32_t stage_cells) const
-{
-    for (const StepList& l : steps)
-        if (steps2d_smem(l.floats, stage_cells) > kPlaneMaxSmem) return false;
-    return true;
-}
+bool Diffusion::steps_fit(uint32_t stage_cells) const { return steps2d_smem(steps.floats, stage_cells) <= kPlaneMaxSmem; }
 
 int Diffusion::steps_2d(int n, bool faces, const RunArgs& runs, uint32_t stage_cells)
 {
     for (int s = 0; s < n; s += kMaxFusedSteps) {
         const int k = std::min(kMaxFusedSteps, n - s);
-        for (const StepList& l : steps) {
-            cudaError_t e = launch_steps2d(ctx->stream, l.cls, planes[0].jobs.as<PlaneJob>(), planes[0].n, tab.as<float>(), tmaps.p,
-                                           l.floats, runs, k, faces ? 1 : 0, stage_cells, ctx->status);
-            if (e != cudaSuccess) return cuda_fail(ctx, e, "2-D steps launch");
-            ctx->launches++;
-        }
+        cudaError_t e = launch_steps2d(ctx->stream, steps.cls, planes[0].jobs.as<PlaneJob>(), planes[0].n, tab.as<float>(), tmaps.p,
+                                       steps.floats, runs, k, faces ? 1 : 0, stage_cells, ctx->status);
+        if (e != cudaSuccess) return cuda_fail(ctx, e, "2-D steps launch");
+        ctx->launches++;
     }
     return PCG_OK;
 }
@@ -1351,8 +1342,6 @@ int Cells::create(pcg_ctx* c, uint32_t maxc, uint32_t rate_capacity, uint32_t n_
     for (DevBuf* b : {&keys, &vals, &skeys, &sorder, &ktmp, &vtmp})
         PCG_CU(ctx, b->alloc((static_cast<size_t>(max_cells) + 1) * sizeof(uint32_t)));
     PCG_CU(ctx, run_word.alloc((static_cast<size_t>(max_cells) + 1) * sizeof(uint64_t)));
-    PCG_CU(ctx, inst_run.alloc(h_inst.size() * sizeof(uint32_t)));
-    PCG_CU(ctx, cudaMemsetAsync(inst_run.p, 0, inst_run.bytes, ctx->stream));
     PCG_CU(ctx, so_prepare(max_cells));
     max_tiles = so_max_tiles(max_cells, static_cast<uint32_t>(h_inst.size()));
     PCG_CU(ctx, tiles.alloc(static_cast<size_t>(max_tiles) * sizeof(SegTile)));
@@ -1490,7 +1479,7 @@ int Cells::build_order(uint64_t total_vox)
                                      max_cells, inst.as<CellInst>(), has_active ? active.as<uint8_t>() : nullptr,
                                      cell_inst.as<uint32_t>(), invalid_key, keys.as<uint32_t>(), ktmp.as<uint32_t>(),
                                      vtmp.as<uint32_t>(), skeys.as<uint32_t>(), sorder.as<uint32_t>(), sort_scr.p,
-                                     ktmp.as<uint32_t>() + n, vals.as<uint32_t>(), run_word.as<uint64_t>(), inst_run.as<uint32_t>(), run_scr.p,
+                                     ktmp.as<uint32_t>() + n, vals.as<uint32_t>(), run_word.as<uint64_t>(), run_scr.p,
                                      consts ? coef_cells.as<double>() : nullptr, coef.as<double>(), cap,
                                      coef_flags.as<uint32_t>());
     if (e != cudaSuccess) return cuda_fail(ctx, e, "secretion order");
@@ -1560,7 +1549,6 @@ RunArgs Cells::run_args() const
     a.run_start = vals.as<uint32_t>();
     a.run_word = run_word.as<uint64_t>();
     a.n_runs = ktmp.as<uint32_t>() + n;
-    a.inst_run = inst_run.as<uint32_t>();
     a.insts = inst.as<CellInst>();
     a.cs = coef.as<double>();
     a.cap = rates.bytes / (4 * sizeof(double));
@@ -1574,7 +1562,7 @@ uint64_t Cells::device_bytes() const
            keys.bytes + vals.bytes +
            skeys.bytes + sorder.bytes + ktmp.bytes + vtmp.bytes + sort_scr.bytes + tiles.bytes + inst_tile.bytes +
            run_scr.bytes +
-           run_word.bytes + inst_run.bytes;
+           run_word.bytes;
 }
 
 // ------------------------------------------------------------------ mechanics

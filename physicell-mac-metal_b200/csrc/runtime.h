@@ -173,8 +173,10 @@ struct PlaneList {
     uint64_t units = 0;        // voxel-substrates covered
 };
 
-// 2-D planes that take several sub-steps in one launch (k_steps_2d).
-struct StepList {
+// A single 2-D simulation's planes taking several sub-steps in one launch
+// (k_steps_2d).
+struct FusedSteps {
+    bool on = false;
     int cls = 0;               // steps2d_class
     uint32_t floats = 0;       // plane_floats of the planes
 };
@@ -208,8 +210,7 @@ public:
     // x-z plane (zplanes); rest[2] holds the z tiles of the others.
     std::vector<PlaneList> zplanes;
     std::vector<SweepList> rest[3];
-    // A single 2-D simulation's planes again, for steps_2d().
-    std::vector<StepList> steps;
+    FusedSteps steps;                  // on: planes[0] holds the simulation's planes
     bool use_planes = true;            // set before build()
     std::string shapes;
 
@@ -222,13 +223,12 @@ public:
     int sweep(int axis, bool fuse_faces, const uint8_t* mask);
     int sweeps(bool fuse_faces, const uint8_t* mask);
     // n sub-steps (sweeps, with faces the Dirichlet reset, with run_word the
-    // secretion) of every instance in 'steps'; side streams as launch_planes
-    // stage_cells: the most cells of an instance, whose runs and terms are
-    // staged in shared memory (steps_fit; 0 without secretion)
+    // secretion) of the single 2-D simulation, on the context stream;
+    // stage_cells: its cells, whose runs and terms are staged in shared memory
+    // (steps_fit; 0 without secretion)
     int steps_2d(int n, bool faces, const RunArgs& runs, uint32_t stage_cells);
-    bool steps_fit(uint32_t stage_cells) const;   // they fit beside every plane
-    // one launch of steps_2d is the way to take n sub-steps of every instance
-    bool takes_steps(int n) const;
+    bool steps_fit(uint32_t stage_cells) const;   // they fit beside a plane
+    bool takes_steps(int n) const;                // steps_2d is the way to take n sub-steps
     int dirichlet();
     int gradients(float* gx, float* gy, float* gz);   // device arrays of total_vox_sub floats, dense per instance
     int upload(uint32_t i, const float* host, bool async_pinned = false);
@@ -305,7 +305,6 @@ public:
     // (rebuilt with the instance table), so_passes x so_bits the digits.
     DevBuf keys, vals, skeys, sorder, ktmp, vtmp, sort_scr, run_scr, tiles, inst_tile;
     DevBuf run_word;   // per run: instance and density element of its voxel (make_run_word)
-    DevBuf inst_run;   // per instance with secreting cells: its first run
     uint32_t invalid_key = 0;
     uint32_t ntiles = 0, max_tiles = 0, n_inst_tiled = 0;
     int so_passes = 1, so_bits = 0;

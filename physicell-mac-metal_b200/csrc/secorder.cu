@@ -326,8 +326,6 @@ __global__ void __launch_bounds__(kThreads) k_so_scatter(const SegTile* __restri
 // k_so_run_write numbers the tile's heads (ballots, then the 64 warp-row
 // counts in order) and writes the runs.  Run r starts at run_start[r] and
 // ends at run_start[r + 1] (run_start[n_runs] = n, *n_runs = the count).
-// An instance with secreting cells gets the index of its first run (inst_run;
-// the entry of one without is left as it was).
 // A run of secreting cells gets one word: its instance and the density
 // element of its voxel (substrate 0, padded rows); a run of non-secreting
 // cells gets kRunNone.
@@ -365,8 +363,7 @@ __global__ void __launch_bounds__(kThreads) k_so_run_write(const uint32_t* __res
                                                            const uint32_t* __restrict__ cell_inst,
                                                            const CellInst* __restrict__ insts,
                                                            uint32_t* __restrict__ run_start,
-                                                           uint64_t* __restrict__ run_word, uint32_t* __restrict__ n_runs,
-                                                           uint32_t* __restrict__ inst_run)
+                                                           uint64_t* __restrict__ run_word, uint32_t* __restrict__ n_runs)
 {
     if (!await_predecessors()) return;
     dependents_may_launch();
@@ -415,7 +412,6 @@ __global__ void __launch_bounds__(kThreads) k_so_run_write(const uint32_t* __res
             const CellInst& in = insts[ii];
             const uint32_t v = key[k] - in.vox_base;
             elem = in.dens_off + static_cast<uint64_t>(v / in.nx) * in.px + v % in.nx;
-            if (p == in.cell_off) inst_run[ii] = r;   // secreting cells fill the start of the instance's range
         }
         run_word[r] = make_run_word(ii, elem);
     }
@@ -495,8 +491,7 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
     k_so_cluster(const SegTile* __restrict__ tiles, const float* __restrict__ soa, uint32_t stride, uint32_t n, int passes,
                  int digit_bits, const CellInst* __restrict__ insts, const uint8_t* __restrict__ active,
                  uint32_t invalid_key, uint32_t* __restrict__ skeys, uint32_t* __restrict__ sorder,
-                 uint32_t* __restrict__ run_start, uint64_t* __restrict__ run_word, uint32_t* __restrict__ n_runs,
-                 uint32_t* __restrict__ inst_run)
+                 uint32_t* __restrict__ run_start, uint64_t* __restrict__ run_word, uint32_t* __restrict__ n_runs)
 {
     constexpr uint32_t kOwn = ClusterSmem<I>::kOwn;
     extern __shared__ __align__(16) unsigned char so_smem[];
@@ -655,7 +650,6 @@ __global__ void __cluster_dims__(kClusterCtas, 1, 1) __launch_bounds__(kClusterT
             if (sec) {
                 const uint32_t row = kk[r] / in.nx;
                 elem = in.dens_off + static_cast<uint64_t>(row) * in.px + (kk[r] - row * in.nx);
-                if (p == 0) inst_run[ii] = q;
             }
             run_word[q] = make_run_word(sec ? ii : kRunNone, elem);
         }
@@ -735,7 +729,7 @@ cudaError_t launch_sec_order(cudaStream_t st, const SegTile* tiles, uint32_t nti
                              int digit_bits, const float* soa, uint32_t stride, const CellInst* insts,
                              const uint8_t* active, const uint32_t* cell_inst, uint32_t invalid_key, uint32_t* keys,
                              uint32_t* ktmp, uint32_t* vtmp, uint32_t* skeys, uint32_t* sorder, void* scratch,
-                             uint32_t* n_runs, uint32_t* run_start, uint64_t* run_word, uint32_t* inst_run, void* run_scratch,
+                             uint32_t* n_runs, uint32_t* run_start, uint64_t* run_word, void* run_scratch,
                              const double* cc, double* cs, uint32_t cap, const uint32_t* flags)
 {
     if (n == 0 || ntiles == 0) return cudaSuccess;
@@ -744,7 +738,7 @@ cudaError_t launch_sec_order(cudaStream_t st, const SegTile* tiles, uint32_t nti
         const uint32_t per = (n + kClusterCtas * kClusterThreads - 1) / (kClusterCtas * kClusterThreads);
         auto run = [&](auto kernel, size_t smem) {
             return launch_chained(st, kernel, kClusterCtas, kClusterThreads, smem, tiles, soa, stride, n, passes, digit_bits,
-                                  insts, active, invalid_key, skeys, sorder, run_start, run_word, n_runs, inst_run);
+                                  insts, active, invalid_key, skeys, sorder, run_start, run_word, n_runs);
         };
         const cudaError_t e = per <= 1   ? run(k_so_cluster<1>, sizeof(ClusterSmem<1>))
                               : per <= 2 ? run(k_so_cluster<2>, sizeof(ClusterSmem<2>))
@@ -794,7 +788,7 @@ cudaError_t launch_sec_order(cudaStream_t st, const SegTile* tiles, uint32_t nti
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
     if ((e = scan_exclusive(st, tile_cnt, tile_off, rt, rscr)) != cudaSuccess) return e;
     launch_chained(st, k_so_run_write, rt, kThreads, 0, skeys, sorder, n, invalid_key, tile_off, tile_cnt, rt, cell_inst, insts,
-                                             run_start, run_word, n_runs, inst_run);
+                                             run_start, run_word, n_runs);
     return cudaGetLastError();
 }
 

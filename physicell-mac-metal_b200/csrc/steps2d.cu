@@ -162,7 +162,7 @@ struct StagedRuns {
 };
 
 __device__ __forceinline__ void stage_runs(StagedRuns& sr, uint32_t* count, uint32_t P, uint32_t ii, uint32_t sub,
-                                           uint32_t r0, uint32_t nruns, const RunArgs& a)
+                                           uint32_t nruns, const RunArgs& a)
 {
     const CellInst& in = a.insts[ii];
     const uint32_t S = in.S, px = in.px, T = blockDim.x, off0 = in.cell_off;
@@ -171,14 +171,14 @@ __device__ __forceinline__ void stage_runs(StagedRuns& sr, uint32_t* count, uint
     sr.f = a.flags[ii];
     if (threadIdx.x == 0) *count = 0;
     __syncthreads();
-    for (uint32_t r = r0 + threadIdx.x; r < nruns; r += T) {
+    for (uint32_t r = threadIdx.x; r < nruns; r += T) {
         const uint64_t w = a.run_word[r];
         const uint32_t p0 = a.run_start[r], p1 = a.run_start[r + 1];
         if (static_cast<uint32_t>(w >> kRunDensBits) != ii) break;
-        sr.place[r - r0] = plane_place(static_cast<uint32_t>((w & kRunDensMask) - in.dens_off), px, inv_px, P);
-        sr.start[r - r0] = p0 - off0;
-        sr.start[r - r0 + 1] = p1 - off0;   // the next run's thread writes the same
-        atomicMax(count, r - r0 + 1);
+        sr.place[r] = plane_place(static_cast<uint32_t>((w & kRunDensMask) - in.dens_off), px, inv_px, P);
+        sr.start[r] = p0 - off0;
+        sr.start[r + 1] = p1 - off0;   // the next run's thread writes the same
+        atomicMax(count, r + 1);
         for (uint32_t q = p0 - off0; q < p1 - off0; ++q) {
             const uint64_t o = static_cast<uint64_t>(q) * S;
             const double c2 = c0a[2 * a.cap + o];
@@ -266,14 +266,10 @@ __global__ void __launch_bounds__(kSteps2dThreads) k_steps_2d(const PlaneJob* __
         bulk_load(tx, tab + jb.tab_x, tbx, bar);
         bulk_load(ty, tab + jb.tab_y, tby, bar);
     }
-    // the instance's first run, if it has secreting cells (else the entry
-    // names another instance's run, or none)
-    uint32_t r0 = 0, nruns = 0;
-    if (a.run_word) {
-        r0 = a.inst_run[ii];
-        nruns = *a.n_runs;
-        if (r0 >= nruns || static_cast<uint32_t>(a.run_word[r0] >> kRunDensBits) != ii) nruns = 0;
-    }
+    // the runs, if any cell secretes (the first one is then a voxel's: those
+    // of non-secreting cells come last)
+    uint32_t nruns = 0;
+    if (a.run_word && static_cast<uint32_t>(a.run_word[0] >> kRunDensBits) == ii) nruns = *a.n_runs;
     bool got;
     if (status[1] & PCG_DEV_TEST_GIVE_UP) {   // test switch: this wait's bound ran out
         if (threadIdx.x == 0) atomicOr(status, PCG_DEV_TIMEOUT);
@@ -303,7 +299,7 @@ __global__ void __launch_bounds__(kSteps2dThreads) k_steps_2d(const PlaneJob* __
         sr.cap = stage_cells;
         sr.start = reinterpret_cast<uint32_t*>(sr.terms + kStageTerms * static_cast<size_t>(stage_cells));
         sr.place = sr.start + stage_cells + 1;
-        stage_runs(sr, reinterpret_cast<uint32_t*>(smem + 64), P, ii, jb.sub, r0, nruns, a);
+        stage_runs(sr, reinterpret_cast<uint32_t*>(smem + 64), P, ii, jb.sub, nruns, a);
     }
     for (int step = 0; step < n_steps; ++step) {
         lane_lines<R, true>(pl, static_cast<int>(P), ny, rx, tx);
