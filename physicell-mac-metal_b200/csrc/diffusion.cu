@@ -53,12 +53,10 @@ __device__ __forceinline__ LineRule rule_of(const SweepTile& t)
     LineRule r;
     r.tab = t.tab;
     r.n = t.n;
-    r.c = 0.f;
     r.fold = t.fold;
     r.T = t.T;
     r.dir = t.inst >> 31;
     r.inst = t.inst & 0x7fffffffu;
-    r._pad = 0;
     return r;
 }
 

@@ -34,12 +34,10 @@ enum Field : int {
 struct LineRule {
     uint32_t tab;   // first float of the rule's table (multiple of 8)
     uint32_t n;     // line length
-    float c;        // D dt / h^2
     float fold;     // Dirichlet RHS fold: c T (2 c T when n == 3), 0 without Dirichlet
     float T;        // Dirichlet target
     uint32_t dir;   // Dirichlet enabled
     uint32_t inst;  // instance index (step mask lookup)
-    uint32_t _pad;
 };
 
 // Longest line the split tables serve (tensor-map boxes are at most 256).
@@ -86,10 +84,9 @@ struct SweepTile {
     uint32_t i0;       // x index of the tile's first column (column tiles)
     uint32_t nx;       // the instance's nx
     uint32_t face;     // TILE_FACE: the Dirichlet reset is fused into this sweep;
-                       // TILE_ROWS: x tile; TILE_TENSOR: moved with tensor map 'map';
-                       // TILE_AXIS_Z: z tile (else y)
+                       // TILE_ROWS: x tile; TILE_AXIS_Z: z tile (else y)
     uint32_t outer;    // column tiles: first slab (k for y, j for z); row tiles: first line
-    uint32_t map;      // index of the 128-byte tensor map
+    uint32_t map;      // index of the 128-byte tensor map (not read by k_sweep_long)
     uint16_t width;    // columns per slab (column tiles): 32, 16 or 8
     uint16_t nslab;    // slabs in the tile
     uint32_t outer_n;  // number of slabs (nz for y, ny for z)
@@ -102,7 +99,7 @@ struct SweepTile {
     uint32_t inst;     // instance index; bit 31 set: Dirichlet
 };
 static_assert(sizeof(SweepTile) == 64, "one 64-byte descriptor per tile");
-enum : uint32_t { TILE_FACE = 1u, TILE_ROWS = 4u, TILE_TENSOR = 8u, TILE_AXIS_Z = 16u };
+enum : uint32_t { TILE_FACE = 1u, TILE_ROWS = 4u, TILE_AXIS_Z = 16u };
 
 // Tensor-map slots per rule: x rules use slot 0, y / z rules one per
 // column-tile width (32, 16, 8).
@@ -235,7 +232,7 @@ cudaError_t launch_chained(cudaStream_t st, void (*kernel)(KArgs...), unsigned g
 // (rows).  x-y jobs (z slab k of one instance-substrate): the plane tensor
 // map (box row_smem_pitch(nx) x ny, slot 1 of the x rule), first row
 // row0 = k * ny, x and y rules: every row, then every column is solved.
-// z jobs (kPlaneZ: the x-z plane y = row0, or a strip of it from x = x0): the
+// z jobs (the x-z plane y = row0, or a strip of it from x = x0): the
 // 3-D map of slot 3 of the z rule (box pitch x 1 x nz), nx = the strip's
 // columns, ny = nz, the z rule in the y fields: every column (a z line) is
 // solved.
@@ -245,14 +242,13 @@ struct PlaneJob {
     uint32_t nx, ny;
     uint32_t tab_x, tab_y;   // table offsets (floats)
     float fold_x, T_x, fold_y, T_y;
-    uint32_t inst;           // instance | kPlaneDirX | kPlaneDirY | kPlaneFaces | kPlaneZ | kPlaneSlabFace
+    uint32_t inst;           // instance | kPlaneDirX | kPlaneDirY | kPlaneFaces | kPlaneSlabFace
     uint32_t sub;            // substrate
     uint32_t x0, pitch, full_nx;   // z jobs: first column, columns of the box, the block's nx
     uint32_t _pad;
 };
 static_assert(sizeof(PlaneJob) == 64, "PlaneJob is 64 bytes");
 constexpr uint32_t kPlaneDirX = 1u << 31, kPlaneDirY = 1u << 30, kPlaneFaces = 1u << 29;
-constexpr uint32_t kPlaneZ = 1u << 28;          // an x-z plane of z lines
 constexpr uint32_t kPlaneSlabFace = 1u << 27;   // z job: the plane is a y face of the block
 constexpr uint32_t kPlaneInstMask = (1u << 27) - 1u;
 // Threads of a plane CTA: one per line of the longer side, at most 256.  (A
@@ -313,7 +309,7 @@ constexpr uint32_t kLongLines = 8;
 size_t sweep_tma_smem(int warps, int nstages, int stage_floats);
 int sweep_tma_occupancy(bool rows, int warps, int nstages, int stage_floats);   // CTAs per SM (0 = does not fit)
 // tmaps: the 128-byte CUtensorMaps the tiles name (64-byte aligned, global
-// memory); every tile is flagged TILE_TENSOR.
+// memory).
 // Fused x + y sweeps (z: x-z planes of z lines), one CTA of 'threads' per
 // plane; 'floats' = the largest plane_floats of the jobs, 'ahead' = the L2
 // prefetch distance in jobs.

@@ -381,7 +381,6 @@ int Diffusion::build(pcg_ctx* c, std::vector<DiffInstance> instances)
                 LineRule r{};
                 r.tab = static_cast<uint32_t>(h_tab_.size());
                 r.n = n;
-                r.c = static_cast<float>(cc);
                 r.T = sp.target_value;
                 r.dir = dir ? 1u : 0u;
                 r.inst = static_cast<uint32_t>(i);
@@ -465,10 +464,7 @@ int Diffusion::build(pcg_ctx* c, std::vector<DiffInstance> instances)
     }
     PCG_CU(ctx, dens.alloc(std::max<uint64_t>(dens_elems, 32) * sizeof(float)));
     PCG_CU(ctx, cudaMemsetAsync(dens.p, 0, dens.bytes, ctx->stream));
-    PCG_CU(ctx, rules.alloc(std::max<size_t>(h_rules_.size(), 1) * sizeof(LineRule)));
     PCG_CU(ctx, tab.alloc(std::max<size_t>(h_tab_.size(), 8) * sizeof(float)));
-    if (!h_rules_.empty())
-        PCG_CU(ctx, cudaMemcpyAsync(rules.p, h_rules_.data(), h_rules_.size() * sizeof(LineRule), cudaMemcpyHostToDevice, ctx->stream));
     if (!h_tab_.empty())
         PCG_CU(ctx, cudaMemcpyAsync(tab.p, h_tab_.data(), h_tab_.size() * sizeof(float), cudaMemcpyHostToDevice, ctx->stream));
     // tensor maps, four 128-byte slots per rule (kMapsPerRule): x rules use
@@ -702,7 +698,7 @@ int Diffusion::build_planes()
                         j.tab_y = rz.tab;
                         j.fold_y = rz.fold;
                         j.T_y = rz.T;
-                        j.inst = static_cast<uint32_t>(i) | kPlaneZ | (rz.dir ? (kPlaneDirY | kPlaneFaces) : 0u) |
+                        j.inst = static_cast<uint32_t>(i) | (rz.dir ? (kPlaneDirY | kPlaneFaces) : 0u) |
                                  ((y == 0 || y + 1 == ny) ? kPlaneSlabFace : 0u);
                         zjobs[c].push_back(j);
                     }
@@ -792,7 +788,7 @@ int Diffusion::build_axis(int axis, const std::vector<uint8_t>* skip, std::vecto
                     t.map = rule * kMapsPerRule;
                     t.width = 32;
                     t.nslab = 1;
-                    t.face = TILE_ROWS | (fast ? TILE_TENSOR : 0u);
+                    t.face = TILE_ROWS;
                     out.push_back(t);
                 }
                 nl += lines;
@@ -822,7 +818,6 @@ int Diffusion::build_axis(int axis, const std::vector<uint8_t>* skip, std::vecto
                         t.width = static_cast<uint16_t>(width);
                         t.nslab = static_cast<uint16_t>(std::min(group, outer - o));
                         t.map = rule * kMapsPerRule + static_cast<uint32_t>(w);
-                        if (fast) t.face |= TILE_TENSOR;
                         if (axis == 2) t.face |= TILE_AXIS_Z;
                         if (final_axis && dir) t.face |= TILE_FACE;
                         out.push_back(t);
@@ -1138,7 +1133,7 @@ int Diffusion::fill(uint32_t i, const float* values)
 
 uint64_t Diffusion::device_bytes() const
 {
-    uint64_t b = dens.bytes + rules.bytes + tab.bytes + faces.bytes;
+    uint64_t b = dens.bytes + tab.bytes + faces.bytes;
     for (int a = 0; a < 3; ++a)
         for (const auto& l : lists[a]) b += l.tiles.bytes;
     for (int a = 0; a < 3; ++a)

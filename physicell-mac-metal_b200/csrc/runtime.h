@@ -199,7 +199,7 @@ public:
     uint64_t dens_elems = 0;
     uint64_t total_vox = 0;        // sum nx*ny*nz
     uint64_t total_vox_sub = 0;    // sum nx*ny*nz*S
-    DevBuf dens, rules, tab, faces, grad_jobs, tmaps;
+    DevBuf dens, tab, faces, grad_jobs, tmaps;
     uint32_t n_faces = 0;
     std::vector<SweepList> lists[3];
     // Instances whose x-y planes fit shared memory run their x and y sweeps
