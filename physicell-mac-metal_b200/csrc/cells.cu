@@ -201,9 +201,10 @@ __device__ __forceinline__ void apply_run(float* __restrict__ d, uint64_t pitch,
 // sectors), and in crowded voxels the cells' chain.  So a thread advances
 // several substrates side by side with the next cell's terms in flight and
 // the division as quotient() (as a subroutine it takes 128 cycles and
-// overlaps nothing).  How many depends on the number of runs:
-//   WIDE (launch_secrete's rule): few runs, at most some waves of the GPU:
-//   each thread's own latency counts, so four substrates that only take up,
+// overlaps nothing).  How many depends on the most runs there can be, which
+// the host knows as the number of cells:
+//   WIDE (launch_secrete's rule): few, at most some waves of the GPU: each
+//   thread's own latency counts, so four substrates that only take up,
 //   three with all terms.  90 registers.  A sub-step of 200000 cells on four
 //   substrates 15.4 -> 11.0 us, of 8191 with all terms on three 7.1 -> 3.8.
 //   else: threads in flight count; two substrates that only take up, 40
@@ -819,17 +820,21 @@ cudaError_t launch_sec_permute(cudaStream_t st, const uint32_t* skeys, const uin
 
 cudaError_t launch_secrete(cudaStream_t st, float* dens, const uint32_t* run_start, const uint64_t* run_word,
                            const uint32_t* n_runs, uint32_t max_runs, uint32_t max_s, const CellInst* insts, const double* cs, uint32_t cap,
-                           const uint32_t* flags, const uint8_t* mask, int block)
+                           const uint32_t* flags, const uint8_t* mask, int sms, int block)
 {
     if (max_runs == 0 || max_s == 0) return cudaSuccess;
     if (block < 32 || block > 256 || block % 32) return cudaErrorInvalidValue;
-    // wide up to four waves of the GPU (5 x 128 threads on 148 SMs: 379k
-    // runs), eight from three substrates on, where the other form passes over
-    // the run more than once.  A mechanics period on 100^3 voxels, wide / not:
-    // 400000 cells 333 / 340 us (one substrate), 374 / 414 (two), 570 / 647
-    // (four); 800000 586 / 549, 631 / 626, 942 / 1236
-    constexpr uint32_t kWideRuns = 4u * 148u * 5u * kWideBlock;
-    if (max_runs <= (max_s > 2 ? 2u * kWideRuns : kWideRuns)) {
+    // wide up to four waves of the GPU by cells (5 x 128 threads an SM: 379k
+    // cells on 148 SMs), eight from three substrates on, where the other form
+    // passes over the run more than once.  A mechanics period on 100^3 voxels,
+    // wide / not: 400000 cells 333 / 340 us (one substrate), 374 / 414 (two),
+    // 570 / 647 (four); 800000 586 / 549, 631 / 626, 942 / 1236.  A crowded
+    // store has fewer runs than cells and could gain from the wide form past
+    // the line (10^6 cells in 4320 voxels, all terms, three substrates: 134 us
+    // against 417), a uniform one of more cells than voxels would lose (10^6
+    // in 60^3, uptake of one: 9.1 against 6.8); the host cannot tell them apart.
+    const uint32_t wide_cells = 4u * 5u * kWideBlock * static_cast<uint32_t>(sms);
+    if (max_runs <= (max_s > 2 ? 2u * wide_cells : wide_cells)) {
         const int wide = std::min(block, kWideBlock);
         return launch_chained(st, k_secrete<true>, blocks_for(max_runs, wide), wide, 0, dens, run_start, run_word, n_runs,
                               insts, cs, cap, flags, mask);
@@ -911,15 +916,14 @@ cudaError_t mech_forces_prepare()
 cudaError_t launch_mech_forces(cudaStream_t st, const float4* spos, const float4* sprm,
                                const uint32_t* start, uint32_t n, const uint32_t* cell_inst,
                                const CellInst* insts, const uint32_t* reach, float* soa, uint32_t stride,
-                               uint32_t* diag_cnt, uint32_t* diag_hash, const uint8_t* mask, ForceShape shape)
+                               uint32_t* diag_cnt, uint32_t* diag_hash, const uint8_t* mask, ForceShape shape, int sms)
 {
     if (n == 0) return cudaSuccess;
     if (shape.block < 32 || shape.block > 256 || shape.block % 32 != 0) return cudaErrorInvalidValue;
     const unsigned grid = blocks_for(n, shape.block);
     const bool dg = diag_cnt != nullptr;
-    // wide up to two waves of the GPU (3 x 256 threads on 148 SMs)
-    constexpr uint32_t kWideCells = 2u * 148u * 3u * 256u;
-    if (shape.queue == 0 && !dg && n <= kWideCells)
+    // wide up to two waves of the GPU (3 x 256 threads an SM)
+    if (shape.queue == 0 && !dg && n <= 2u * 3u * 256u * static_cast<uint32_t>(sms))
         return forces_variant<0, false, true>(st, grid, shape.block, spos, sprm, start, n, cell_inst, insts, reach, soa, stride,
                                               diag_cnt, diag_hash, mask);
 #define PCG_FORCES(Q)                                                                                                \

@@ -364,14 +364,14 @@ cudaError_t launch_sec_cell_consts(cudaStream_t st, const float* soa, uint32_t s
 cudaError_t launch_sec_permute(cudaStream_t st, const uint32_t* skeys, const uint32_t* sorder, uint32_t n,
                                const uint32_t* cell_inst, const CellInst* insts, uint32_t invalid_key,
                                const uint32_t* flags, const double* cc, uint32_t n_rate, double* cs);
-// n_runs: device count (heads_rid[n]); max_runs >= it; max_s = largest S;
+// n_runs: device count; max_runs >= it; max_s = largest S; sms: the GPU's SMs;
 // runs whose word names kRunNone are skipped.
 // cs: constants c0, c1, c2 as three arrays of cap; flags: per instance, bit 0
 // some c0 not +0, bit 1 some c1 not +0 (written by launch_sec_cell_consts).
 cudaError_t launch_secrete(cudaStream_t st, float* dens, const uint32_t* run_start, const uint64_t* run_word,
                            const uint32_t* n_runs,
                            uint32_t max_runs, uint32_t max_s, const CellInst* insts, const double* cs, uint32_t cap,
-                           const uint32_t* flags, const uint8_t* mask, int block = 256);
+                           const uint32_t* flags, const uint8_t* mask, int sms, int block = 256);
 
 // Mechanics binning as a counting sort: launch_mech_bin writes each cell's
 // global mechanics-voxel key, counts it (counts: V + 1 zeroed words) and
@@ -407,7 +407,7 @@ cudaError_t launch_mech_forces(cudaStream_t st, const float4* spos, const float4
                                const uint32_t* start, uint32_t n,
                                const uint32_t* cell_inst, const CellInst* insts, const uint32_t* reach, float* soa,
                                uint32_t stride, uint32_t* diag_cnt, uint32_t* diag_hash, const uint8_t* mask,
-                               ForceShape shape);
+                               ForceShape shape, int sms);
 // Copies of a removal plan: (dst, src) pairs, each cell's 28 SoA fields,
 // 4 x S rates (arrays of rate_cap doubles, [cell * S + s]), active flag and
 // three FP64 master positions (arrays of stride doubles; pos64 may be null).

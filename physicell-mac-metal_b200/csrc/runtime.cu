@@ -1531,7 +1531,7 @@ int Cells::secrete(Diffusion& d, const uint8_t* mask)
                                    ktmp.as<uint32_t>() + n, n, max_s,
                                    inst.as<CellInst>(), coef.as<double>(),
                                    static_cast<uint32_t>(rates.bytes / (4 * sizeof(double))),
-                                   coef_flags.as<uint32_t>(), mask, sec_block);
+                                   coef_flags.as<uint32_t>(), mask, ctx->sms, sec_block);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "secretion launch");
     if (n && max_s) ctx->launches++;
     return PCG_OK;
@@ -1633,7 +1633,7 @@ int Mechanics::force_pass(Cells& c, const uint8_t* mask)
     cudaStream_t st = ctx->stream;
     cudaError_t e = launch_mech_forces(st, spos.as<float4>(), sprm.as<float4>(), start.as<uint32_t>(), c.n,
                            c.cell_inst.as<uint32_t>(), c.inst.as<CellInst>(), reach(), c.soa.as<float>(), c.max_cells, diag ? dcnt.as<uint32_t>() : nullptr, diag ? dhash.as<uint32_t>() : nullptr,
-                           mask, fshape);
+                           mask, fshape, ctx->sms);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "forces launch");
     ctx->launches++;
     return PCG_OK;
