@@ -269,7 +269,11 @@ __global__ void __launch_bounds__(kSteps2dThreads) k_steps_2d(const PlaneJob* __
     // the runs, if any cell secretes (the first one is then a voxel's: those
     // of non-secreting cells come last)
     uint32_t nruns = 0;
-    if (a.run_word && static_cast<uint32_t>(a.run_word[0] >> kRunDensBits) == ii) nruns = *a.n_runs;
+    if (a.run_word) {
+        const uint64_t w = a.run_word[0];
+        nruns = *a.n_runs;
+        if (static_cast<uint32_t>(w >> kRunDensBits) != ii) nruns = 0;
+    }
     bool got;
     if (status[1] & PCG_DEV_TEST_GIVE_UP) {   // test switch: this wait's bound ran out
         if (threadIdx.x == 0) atomicOr(status, PCG_DEV_TIMEOUT);
