@@ -387,11 +387,12 @@ __global__ void __launch_bounds__(256, 3)
 
 // Lines too long for a tensor box (and any line without a tensor map): one
 // warp per line, kLongLines lines per CTA (8 adjacent columns: one 32-byte
-// sector per row), 'parts' CTAs per tile of up to 32 lines.  Both recurrences are affine, d_i = g_i d_{i-1} + h_i and
-// x_i = g_i x_{i+1} + d_i, so lane l takes K consecutive positions, runs
-// them from zero, the 32 (product of g, end value) pairs are scanned with
-// shuffles, and the lane runs its positions again from the value the scan
-// gives it: 4 K + 10 dependent steps where one thread per line has 2 n.
+// sector per row), 2^log_parts CTAs per tile of up to 32 lines.  Both
+// recurrences are affine, d_i = g_i d_{i-1} + h_i and x_i = g_i x_{i+1} +
+// d_i, so lane l takes K consecutive positions, runs them from zero, the 32
+// (product of g, end value) pairs are scanned with shuffles, and the lane
+// runs its positions again from the value the scan gives it: 4 K + 10
+// dependent steps where one thread per line has 2 n.
 // Values and tables are staged in shared memory with one pad per K
 // positions, so that the lanes' runs hit different banks, and a line's g
 // and values stay in registers between the passes.  A line longer than one
@@ -400,20 +401,39 @@ __global__ void __launch_bounds__(256, 3)
 //
 // What bounds it: the latency of those steps and of one round trip to
 // memory.  A diffusion step (x and y) of 701 x 530 voxels, two substrates,
-// takes 16.4 us, where one thread per line in place (n dependent,
+// takes 14.2 us, where one thread per line in place (n dependent,
 // uncoalesced accesses) took 516; the x sweep of 300-voxel lines (2 x 300 x
-// 300 x 60) 95 us, where 32-line tiles with bulk row copies took 335.
+// 300 x 60) 95 us, where 32-line tiles with bulk row copies took 335.  The
+// check for values that are not finite costs 1 to 2 %; within the register
+// bound below, since the fourth block of an SM goes at 65 registers and with it
+// a fifth of the rate (300^3: 385 -> 465 us).
 template <int K>
 __host__ __device__ constexpr int long_stride() { return 32 * (K + 1) + 4; }   // 4 mod 32: 8 columns hit 8 bank groups
 
 template <int K>
 __device__ __forceinline__ int long_at(int i) { return i + i / K; }
 
-// Inclusive scan of a segment's affine maps (D, G) over the lanes, in walking
-// order; 'term' gives one map's G a + D.
-template <bool BACK, class TERM>
-__device__ __forceinline__ void scan_maps(float& D, float& G, int pos, TERM term)
+// One direction of a line's segment: v[k] = h (forward) or d (backward) in,
+// the recurrence's values out; 'edge' enters at the segment's first
+// position in walking order.  Returns the value at the last one.
+//   The product G of many g below 1 underflows to 0, and 0 times an infinite
+// value would be NaN where a walk position by position carries it on undamped.
+// WILD: an infinite a is multiplied by 'one' instead: 1, or 0 where the rule
+// has no coupling and every g is 0.  finite: the lane's scanned value is (an
+// infinite or NaN value anywhere on a segment leaves some lane's not finite).
+template <int K, bool BACK, bool WILD>
+__device__ __forceinline__ float long_scan(float (&v)[K], const float (&g)[K], float edge, float one, bool& finite, int lane)
 {
+    auto term = [one](float m, float a, float d) { return fmaf(WILD && fabsf(a) == INFINITY ? one : m, a, d); };
+    float D = 0.f, G = 1.f;
+#pragma unroll
+    for (int q = 0; q < K; ++q) {
+        const int k = BACK ? K - 1 - q : q;
+        D = fmaf(g[k], D, v[k]);
+        G *= g[k];
+    }
+    // inclusive scan of the affine maps in walking order
+    const int pos = BACK ? 31 - lane : lane;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const float Dp = BACK ? __shfl_down_sync(0xffffffffu, D, o) : __shfl_up_sync(0xffffffffu, D, o);
@@ -423,41 +443,10 @@ __device__ __forceinline__ void scan_maps(float& D, float& G, int pos, TERM term
             G *= Gp;
         }
     }
-}
-
-// One direction of a line's segment: v[k] = h (forward) or d (backward) in,
-// the recurrence's values out; 'edge' enters at the segment's first
-// position in walking order.  Returns the value at the last one.
-//   The product G of many g below 1 underflows to 0, and 0 times an infinite
-// value would be NaN where a walk position by position carries it on undamped.
-// So where a value is not finite ('wild' is set) the scan is run again with
-// an infinite a multiplied by 'one' instead: 1, or 0 where the rule has no
-// coupling and every g is 0.
-template <int K, bool BACK>
-__device__ __forceinline__ float long_scan(float (&v)[K], const float (&g)[K], float edge, float one, bool& wild, int lane)
-{
-    float D, G;
-    auto run = [&]() {   // the lane's positions from zero
-        D = 0.f;
-        G = 1.f;
-#pragma unroll
-        for (int q = 0; q < K; ++q) {
-            const int k = BACK ? K - 1 - q : q;
-            D = fmaf(g[k], D, v[k]);
-            G *= g[k];
-        }
-    };
-    const int pos = BACK ? 31 - lane : lane;
-    run();
-    scan_maps<BACK>(D, G, pos, [](float m, float a, float d) { return fmaf(m, a, d); });
-    wild = __any_sync(0xffffffffu, !(fabsf(D) < INFINITY) || !(fabsf(edge) < INFINITY));
-    if (wild) {
-        run();
-        scan_maps<BACK>(D, G, pos, [one](float m, float a, float d) { return fmaf(fabsf(a) == INFINITY ? one : m, a, d); });
-    }
+    finite = fabsf(D) < INFINITY;
     const float Dx = BACK ? __shfl_down_sync(0xffffffffu, D, 1) : __shfl_up_sync(0xffffffffu, D, 1);
     const float Gx = BACK ? __shfl_down_sync(0xffffffffu, G, 1) : __shfl_up_sync(0xffffffffu, G, 1);
-    float x = pos == 0 ? edge : fmaf(wild && fabsf(edge) == INFINITY ? one : Gx, edge, Dx);
+    float x = pos == 0 ? edge : term(Gx, edge, Dx);
 #pragma unroll
     for (int q = 0; q < K; ++q) {
         const int k = BACK ? K - 1 - q : q;
@@ -467,21 +456,45 @@ __device__ __forceinline__ float long_scan(float (&v)[K], const float (&g)[K], f
     return __shfl_sync(0xffffffffu, x, BACK ? 0 : 31);
 }
 
+// A line of one segment that holds an infinite or NaN value, from and to the
+// lane's place in the stage (out of line: its registers are not the sweep's).
 template <int K>
-__global__ void __launch_bounds__(32 * kLongLines) k_sweep_long(float* __restrict__ dens,
-                                                                const SweepTile* __restrict__ tiles, uint32_t parts,
+__device__ __noinline__ void long_wild(float* s, const float* sg, const float* si, int n, float fold, float one, int lane)
+{
+    float v[K], g[K];
+    bool finite;
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+        const int i = lane * K + k, at = lane * (K + 1) + k;
+        g[k] = sg[at];
+        v[k] = (s[k] + (i == 1 || i == n - 2 ? fold : 0.f)) * si[at];
+    }
+    long_scan<K, false, true>(v, g, 0.f, one, finite, lane);
+    // the forward walk leaves NaN (0 times infinity) at the end node and past
+    // it, where the way back starts from 0
+#pragma unroll
+    for (int k = 0; k < K; ++k)
+        if (lane * K + k >= n - 1) v[k] = 0.f;
+    long_scan<K, true, true>(v, g, 0.f, one, finite, lane);
+#pragma unroll
+    for (int k = 0; k < K; ++k) s[k] = v[k];
+}
+
+template <int K>
+__global__ void __launch_bounds__(32 * kLongLines, K <= 16 ? 4 : 2) k_sweep_long(float* __restrict__ dens,
+                                                                const SweepTile* __restrict__ tiles, int log_parts,
                                                                 const float* __restrict__ tab, int apply_faces,
                                                                 const uint8_t* __restrict__ mask)
 {
-    if (!await_predecessors()) return;
-    dependents_may_launch();
     constexpr int kSeg = 32 * K, kStride = long_stride<K>();
     extern __shared__ float sh[];
     float* sg = sh + kLongLines * kStride;   // g of the segment's positions
     float* si = sg + kStride;                // 1 / den
-    const SweepTile tile = tiles[blockIdx.x / parts];
-    const uint32_t l0 = blockIdx.x % parts * kLongLines;   // the CTA's first line of the tile
+    const SweepTile tile = tiles[blockIdx.x >> log_parts];   // written once, before any step
+    const uint32_t l0 = (blockIdx.x & ((1u << log_parts) - 1u)) * kLongLines;   // the CTA's first line of the tile
     const LineRule r = rule_of(tile);
+    if (!await_predecessors()) return;
+    dependents_may_launch();
     if (l0 >= tile.count || !tile_on(r, mask)) return;   // the whole CTA leaves together
     const int n = static_cast<int>(r.n), lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const bool rows = (tile.face & TILE_ROWS) != 0;
@@ -525,9 +538,11 @@ __global__ void __launch_bounds__(32 * kLongLines) k_sweep_long(float* __restric
             v[k] = (v[k] + f) * si[lane * (K + 1) + k];
         }
     };
-    auto store = [&](int s0, bool last) {   // interior values (and, at the end, the end nodes' targets and the faces)
+    auto store = [&](int s0, bool last, bool put = true) {   // interior values (and, at the end, the end nodes' targets and the faces)
+        if (put) {
 #pragma unroll
-        for (int k = 0; k < K; ++k) sw[k] = v[k];
+            for (int k = 0; k < K; ++k) sw[k] = v[k];
+        }
         __syncthreads();
         if (mine) {
 #pragma unroll 8
@@ -542,36 +557,31 @@ __global__ void __launch_bounds__(32 * kLongLines) k_sweep_long(float* __restric
         __syncthreads();   // the stage may be loaded again
     };
 
-    const float one = n > 3 && __ldg(t + 1) > 0.f ? 1.f : 0.f;   // g of the first interior node: 0 without coupling
+    bool finite;
+    auto coupled = [&]() { return n > 3 && __ldg(t + 1) > 0.f ? 1.f : 0.f; };   // long_scan's 'one': g of the first interior node
     if (n <= kSeg) {
         load(0);
         to_rhs(0);
-        bool wild;
-        long_scan<K, false>(v, g, 0.f, one, wild, lane);
-        // the forward walk leaves 0 at the end node and past it, but NaN
-        // (0 times infinity) behind an infinite value
-        if (wild) {
-#pragma unroll
-            for (int k = 0; k < K; ++k)
-                if (lane * K + k >= n - 1) v[k] = 0.f;
-        }
-        long_scan<K, true>(v, g, 0.f, one, wild, lane);
-        store(0, true);
+        long_scan<K, false, false>(v, g, 0.f, 0.f, finite, lane);
+        long_scan<K, true, false>(v, g, 0.f, 0.f, finite, lane);
+        const bool wild = __any_sync(0xffffffffu, !finite);
+        if (wild) long_wild<K>(sw, sg, si, n, r.fold, coupled(), lane);
+        store(0, true, !wild);
         return;
     }
+    const float one = coupled();
     float edge = 0.f;
-    bool wild;
     int s0 = 0;
     for (; s0 < n; s0 += kSeg) {
         load(s0);
         to_rhs(s0);
-        edge = long_scan<K, false>(v, g, edge, one, wild, lane);
+        edge = long_scan<K, false, true>(v, g, edge, one, finite, lane);
         store(s0, false);
     }
     edge = 0.f;
     for (s0 -= kSeg; s0 >= 0; s0 -= kSeg) {
         load(s0);
-        edge = long_scan<K, true>(v, g, edge, one, wild, lane);
+        edge = long_scan<K, true, true>(v, g, edge, one, finite, lane);
         store(s0, true);
     }
 }
@@ -826,11 +836,11 @@ cudaError_t launch_sweep_planes(cudaStream_t st, bool z, int threads, const Plan
 }
 
 template <int K>
-static cudaError_t long_variant(cudaStream_t st, float* dens, const SweepTile* tiles, uint32_t ntiles, uint32_t parts,
+static cudaError_t long_variant(cudaStream_t st, float* dens, const SweepTile* tiles, uint32_t ntiles, int log_parts,
                                 const float* tab, int apply_faces, const uint8_t* mask)
 {
     const size_t smem = static_cast<size_t>(kLongLines + 2) * long_stride<K>() * sizeof(float);   // at most 43 KB
-    launch_chained(st, k_sweep_long<K>, ntiles * parts, 32 * kLongLines, smem, dens, tiles, parts, tab, apply_faces, mask);
+    launch_chained(st, k_sweep_long<K>, ntiles << log_parts, 32 * kLongLines, smem, dens, tiles, log_parts, tab, apply_faces, mask);
     return cudaGetLastError();
 }
 
@@ -838,14 +848,14 @@ cudaError_t launch_sweep_long(cudaStream_t st, float* dens, const SweepTile* til
                               const float* tab, int nmax, int apply_faces, const uint8_t* mask)
 {
     if (ntiles == 0) return cudaSuccess;
-    const uint32_t parts = (lines + kLongLines - 1) / kLongLines;
+    const int log_parts = lines <= kLongLines ? 0 : lines <= 2 * kLongLines ? 1 : 2;
     // positions per lane: the fewest that hold the longest line in one
     // segment (a lane's steps, registers and shared memory grow with them),
     // at most 32; longer lines take several segments
-    if (nmax <= 32 * 12) return long_variant<12>(st, dens, tiles, ntiles, parts, tab, apply_faces, mask);
-    if (nmax <= 32 * 16) return long_variant<16>(st, dens, tiles, ntiles, parts, tab, apply_faces, mask);
-    if (nmax <= 32 * 24) return long_variant<24>(st, dens, tiles, ntiles, parts, tab, apply_faces, mask);
-    return long_variant<32>(st, dens, tiles, ntiles, parts, tab, apply_faces, mask);
+    if (nmax <= 32 * 12) return long_variant<12>(st, dens, tiles, ntiles, log_parts, tab, apply_faces, mask);
+    if (nmax <= 32 * 16) return long_variant<16>(st, dens, tiles, ntiles, log_parts, tab, apply_faces, mask);
+    if (nmax <= 32 * 24) return long_variant<24>(st, dens, tiles, ntiles, log_parts, tab, apply_faces, mask);
+    return long_variant<32>(st, dens, tiles, ntiles, log_parts, tab, apply_faces, mask);
 }
 
 cudaError_t launch_dirichlet(cudaStream_t st, float* dens, const FaceJob* jobs, uint32_t njobs)
