@@ -22,6 +22,7 @@ int cuda_fail(pcg_ctx* ctx, cudaError_t e, const char* what)
 {
     std::string m = std::string(what) + ": " + cudaGetErrorName(e) + " (" + cudaGetErrorString(e) + ")";
     if (ctx) ctx->err = m;
+    cudaGetLastError();   // reported here: not again by the next launch's check
     return e == cudaErrorMemoryAllocation ? PCG_ERR_OOM : PCG_ERR_CUDA;
 }
 
