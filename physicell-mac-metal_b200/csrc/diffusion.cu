@@ -19,8 +19,8 @@
 // ones counted from the right end), a 2 x 2 system in the middle, and both
 // halves substituted outwards.  The same operations per value, but two
 // independent chains of n / 2 each way: one thread runs them side by side
-// (split_line), or two threads take one each (half_line).  End nodes keep
-// their value or take the Dirichlet target.
+// (split_line), or two lanes of a warp take one each (lane_half, in the
+// fused 2-D steps).  End nodes keep their value or take the Dirichlet target.
 //
 // Data movement.  density is [s][k][j][i] FP32 with rows padded to a pitch
 // px = nx rounded up to 4 floats, so every row starts on 16 bytes.  Each

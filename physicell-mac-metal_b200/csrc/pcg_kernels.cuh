@@ -475,8 +475,8 @@ cudaError_t radix_sort_pairs(cudaStream_t st, const uint32_t* k_in, const uint32
                              uint32_t* k_out, uint32_t* v_out, uint32_t* k_tmp, uint32_t* v_tmp,
                              uint32_t n, int bits, void* scratch);
 
-// Loads the radix sort's and the scan's kernels on the current device now
-// rather than at their first launch.
+// Loads the radix sort's kernels on the current device now rather than at
+// their first launch.
 cudaError_t sort_kernels_load();
 
 // Exclusive prefix sum of n uint32 values (in may equal out).

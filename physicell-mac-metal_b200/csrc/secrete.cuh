@@ -21,8 +21,8 @@ __device__ __forceinline__ float secrete_terms(float rho32, double c0, double c1
 
 // The quotient a / b rounded as IEEE division rounds it, from y = RN(1 / b),
 // without a call or a branch, so that several run side by side (the
-// compiler's division is a subroutine of some 200 cycles that does not
-// overlap another): two residual corrections of a y give RN(a / b)
+// compiler's division is a subroutine of 128 cycles that does not overlap
+// another): two residual corrections of a y give RN(a / b)
 // (P. Markstein, "Computation of elementary functions on the IBM RISC
 // System/6000 processor", 1990) while nothing over- or underflows: 'ok' is
 // cleared when a (other than +0) or b leaves the range where that is certain.

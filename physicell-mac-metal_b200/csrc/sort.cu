@@ -16,7 +16,8 @@
 //                    (every tile adds up the rows of all tiles itself: at
 //                    most 128 KB of L2 for the 262144 pairs of the static
 //                    sort, less time than a scan of the counts between the
-//                    two launches: 200003 pairs of 20 bits 38.7 -> 30.5 us).
+//                    two launches: 200003 pairs of 20 bits 38.7 -> 30.5 us,
+//                    and 23.1 with one kernel of the chain waiting at a time).
 // Ranks follow input order within a warp, warps follow tile order and
 // tiles follow each other in order, so each pass is stable.
 #include "pcg_kernels.cuh"
@@ -207,8 +208,9 @@ constexpr uint64_t kOneBlock = 4ull * kOneItems * kOneThreads;   // 32768
 // of each group of 4096: all loads are in flight together, the groups' warp
 // scans overlap, and one pass over the 8 x 32 warp totals joins them.  Bound
 // by latency: two round trips to L2 and two barriers, where three launches of
-// the tile kernels pay theirs each (25088 digit counts of a 200 k pair sort:
-// three passes of the sort 49.8 -> 38 us).
+// the tile kernels pay theirs each (the forces of 2000 cells, whose cell-start
+// table has 4356 voxels, 21.6 -> 18.5 us; of 20000 cells in 17576 voxels 29.8
+// -> 27.1, in 29791 27.7 -> 26.3).
 __global__ void __launch_bounds__(kOneThreads) k_scan_one(const uint32_t* __restrict__ in, uint32_t* __restrict__ out,
                                                           uint32_t n)
 {

@@ -14,7 +14,7 @@
 // half, the half's values in registers between the passes; the halves meet
 // through a shuffle.  Longer lines, whose halves would not fit the registers,
 // are solved by one thread each in shared memory (split_line).  10 sub-steps
-// of 50 x 50 voxels: 37.5 -> 16.8 us without cells, 65.5 -> 25.5 with 500,
+// of 50 x 50 voxels: 37.5 -> 16.8 us without cells, 59.2 -> 25.5 with 500,
 // against a plane pass and a secretion launch per sub-step; 181 x 117 with
 // three substrates, no cells: 86.5 -> 52.2.
 #include "lines.cuh"
